@@ -26,6 +26,7 @@ namespace sgc {
 constexpr uint32_t INV = SGC_CSR_INVALID;
 constexpr uint32_t EMPTY = SGC_HASH_EMPTY;
 constexpr uint32_t FULL = 0xFFFFFFFFu;
+constexpr uint32_t NOSLOT = 0xFFFFFFFFu;
 constexpr uint32_t OVF_CAP = SGC_OVERFLOW_CAPACITY;
 constexpr uint32_t TOMB = 0x80000000u;  // tombstone bit of a deleted base-run entry (exact selection)
 
@@ -136,6 +137,22 @@ __device__ __forceinline__ uint32_t ld_cg(const uint32_t* p) { return __ldcg(p);
 __device__ __forceinline__ uint64_t ld_cg(const uint64_t* p) { return __ldcg((const unsigned long long*)p); }
 __device__ __forceinline__ uint4 ld_cg4(const uint32_t* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 
+// Loads of words that only the calling block changes while the kernel runs
+// (stream-order updates): cached in the SM's L1 (CA). Everywhere else the
+// coherent form: L2, where other SMs' changes show.
+template <bool CA>
+__device__ __forceinline__ uint32_t ld_w(const uint32_t* p) {
+    return CA ? *p : __ldcg(p);
+}
+template <bool CA>
+__device__ __forceinline__ uint64_t ld_w(const uint64_t* p) {
+    return CA ? *p : __ldcg((const unsigned long long*)p);
+}
+template <bool CA>
+__device__ __forceinline__ uint4 ld_w4(const uint32_t* p) {
+    return CA ? *reinterpret_cast<const uint4*>(p) : __ldcg(reinterpret_cast<const uint4*>(p));
+}
+
 __device__ __forceinline__ uint32_t pick4(const uint4& q, int k) {
     return k == 0 ? q.x : (k == 1 ? q.y : (k == 2 ? q.z : q.w));
 }
@@ -177,7 +194,7 @@ struct Lanes {
 // scanning in slot order exactly like the reference's serial loop. Loads are
 // 16-byte aligned (col must be 16-byte aligned and padded past the last row
 // to a multiple of 4 slots). Returns false when no slot matches.
-template <int W, class P>
+template <bool CA = false, int W, class P>
 __device__ __forceinline__ bool grp_find(const Lanes<W>& L, const uint32_t* col, uint64_t s, uint64_t e, P pred,
                                          uint64_t& pos, uint32_t& val) {
     constexpr uint64_t R = 4ull * W;  // slots per group-wide 16-byte load
@@ -187,7 +204,7 @@ __device__ __forceinline__ bool grp_find(const Lanes<W>& L, const uint32_t* col,
         for (int k = 0; k < 4; k++) {
             const uint64_t i = c + R * k + 4ull * L.lane;
             q[k] = make_uint4(INV, INV, INV, INV);
-            if (i < e) q[k] = ld_cg4(col + i);
+            if (i < e) q[k] = ld_w4<CA>(col + i);
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -215,7 +232,7 @@ __device__ __forceinline__ bool warp_find(const uint32_t* col, uint64_t s, uint6
 
 // Warp-collective visit of every slot in [s, e): f(slot_index, value) runs on
 // the lane that loaded the slot (each slot once).
-template <class F>
+template <bool CA = false, class F>
 __device__ __forceinline__ void warp_for_each(const uint32_t* col, uint64_t s, uint64_t e, F f) {
     const uint32_t lane = lane_id();
     for (uint64_t c = s & ~3ull; c < e; c += 512) {  // four 16-byte loads per lane in flight
@@ -224,7 +241,7 @@ __device__ __forceinline__ void warp_for_each(const uint32_t* col, uint64_t s, u
         for (int k = 0; k < 4; k++) {
             const uint64_t i = c + 128ull * k + 4ull * lane;
             q[k] = make_uint4(INV, INV, INV, INV);
-            if (i < e) q[k] = ld_cg4(col + i);
+            if (i < e) q[k] = ld_w4<CA>(col + i);
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -245,7 +262,7 @@ __device__ __forceinline__ void warp_for_each(const uint32_t* col, uint64_t s, u
 // round). f(y, arr[y]) runs once per slot. With STOP, the scan ends after the
 // first round in which f returned true on any lane (warp vote); the return
 // value says whether that happened.
-template <bool STOP, int K = 4, class F>
+template <bool STOP, int K = 4, bool CA = false, class F>
 __device__ __forceinline__ bool warp_gather_each(const uint32_t* col, uint64_t s, uint64_t e, uint32_t n,
                                                  const uint32_t* arr, F f) {
     const uint32_t lane = lane_id();
@@ -255,14 +272,14 @@ __device__ __forceinline__ bool warp_gather_each(const uint32_t* col, uint64_t s
         for (int k = 0; k < K; k++) {
             const uint64_t i = c + 128ull * k + 4ull * lane;
             uint4 q = make_uint4(INV, INV, INV, INV);
-            if (i < e) q = ld_cg4(col + i);
+            if (i < e) q = ld_w4<CA>(col + i);
             y[4 * k + 0] = (i + 0 >= s && i + 0 < e) ? q.x : INV;
             y[4 * k + 1] = (i + 1 >= s && i + 1 < e) ? q.y : INV;
             y[4 * k + 2] = (i + 2 >= s && i + 2 < e) ? q.z : INV;
             y[4 * k + 3] = (i + 3 >= s && i + 3 < e) ? q.w : INV;
         }
 #pragma unroll
-        for (int t = 0; t < 4 * K; t++) w[t] = y[t] < n ? ld_cg(arr + y[t]) : 0u;
+        for (int t = 0; t < 4 * K; t++) w[t] = y[t] < n ? ld_w<CA>(arr + y[t]) : 0u;
         bool hit = false;
 #pragma unroll
         for (int t = 0; t < 4 * K; t++)
@@ -290,8 +307,9 @@ __device__ __forceinline__ uint32_t row_len(const Dev& g, uint32_t x) {
 
 // End of the slots of row x that scans visit, [s, s + hw), clamped to the
 // row's capacity (a larger mark sets ERR_ROW).
+template <bool CA = false>
 __device__ __forceinline__ uint64_t live_end(const Dev& g, uint32_t x, uint64_t s) {
-    const uint64_t e = s + ld_cg(g.hw + x), cap = g.rp[x + 1];
+    const uint64_t e = s + ld_w<CA>(g.hw + x), cap = g.rp[x + 1];
     if (e <= cap) return e;
     if ((lane_id() & 15u) == 0) atomicOr(g.err, ERR_ROW);  // the first lane of each half-warp group
     return cap;
@@ -331,13 +349,13 @@ __device__ __forceinline__ bool pristine(const Dev& g, uint32_t x) {
 // Group-collective W-ary search for `key` in the ascending run col[s, e):
 // each round probes W evenly spaced slots and keeps the bucket holding the
 // last probe <= key. Returns the slot index, or ~0 when key is absent.
-template <int W>
+template <bool CA = false, int W>
 __device__ __forceinline__ uint64_t grp_bsearch(const Lanes<W>& L, const uint32_t* col, uint64_t s, uint64_t e,
                                                 uint32_t key) {
     uint64_t lo = s, hi = e;
     while (hi - lo > W) {
         const uint64_t step = (hi - lo) / W;
-        const uint32_t v = ld_cg(col + lo + L.lane * step);
+        const uint32_t v = ld_w<CA>(col + lo + L.lane * step);
         const uint32_t b = L.ballot(v <= key);
         if (!b) return ~0ull;
         const uint32_t top = 31 - __clz(b);
@@ -346,7 +364,7 @@ __device__ __forceinline__ uint64_t grp_bsearch(const Lanes<W>& L, const uint32_
         lo = nlo;
     }
     const uint64_t i = lo + L.lane;
-    const bool hit = i < hi && ld_cg(col + i) == key;
+    const bool hit = i < hi && ld_w<CA>(col + i) == key;
     const uint32_t b = L.ballot(hit);
     return b ? lo + (__ffs(b) - 1) : ~0ull;
 }
@@ -427,18 +445,36 @@ __device__ __forceinline__ bool grp_run_remove(const Lanes<W>& L, const Dev& g, 
     return old == nbr;
 }
 
+// A row without a free slot (one lane): the entry goes to the overflow buffer
+// (the counter always advances, the entry is stored only below capacity); the
+// no-overflow ablation drops it.
+__device__ __forceinline__ void append_overflow(const Dev& g, uint32_t x, uint32_t nbr) {
+    if (g.abl & ABL_NO_OVERFLOW) {
+        g.gctl[graph_of(g, x)].dropped = 1u;
+    } else {
+        const uint32_t pos = atomicAdd(g.ovf_count, 1u);
+        if (pos < OVF_CAP) {
+            g.ovf[pos].local_vertex_idx = x;
+            g.ovf[pos].neighbor_global = nbr;
+        } else {
+            atomicAdd(g.ovf_lost, 1ull);
+            g.gctl[graph_of(g, x)].dropped = 1u;
+        }
+    }
+    flag_asym(g, x);
+}
+
 // add_local_neighbor: claim the first INV slot unless `nbr` shows up first;
-// a full row appends to the overflow buffer (counter always advances, entry
-// stored only below capacity). The row's bounds, base run and high-water
+// a full row appends to the overflow buffer. The row's bounds, base run and high-water
 // mark are read together up front (a mark read early is only lower: the
 // fallback scan to the row's end covers what it misses).
 template <int W>
-__device__ __forceinline__ int grp_add_slot(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr, bool exact) {
+__device__ __forceinline__ int grp_add_slot(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr) {
     const uint64_t s = g.rp[x], e = g.rp[x + 1];
-    const uint32_t bl = (!exact && g.blen) ? ld_cg(g.blen + x) : 0u;
+    const uint32_t bl = g.blen ? ld_cg(g.blen + x) : 0u;
     const uint32_t hw0 = ld_cg(g.hw + x);
     uint64_t from = s;
-    if (!exact && g.blen) {
+    if (g.blen) {
         if (bl) {
             const int r = grp_run_add(L, g, x, nbr, s, bl);
             if (r >= 0) return r;
@@ -449,8 +485,7 @@ __device__ __forceinline__ int grp_add_slot(const Lanes<W>& L, const Dev& g, uin
         // else at the first INV right after the base run.
         const uint64_t len = live_end(g, x, s) - s;
         if (grp_bsearch(L, g.col, s, s + len, nbr) != ~0ull) return ADD_PRESENT;
-        // Past the sorted run: in stream order nothing else changes the row; in
-        // a concurrent batch the updates of this edge are ordered, so nbr can
+        // Past the sorted run: the updates of this edge are ordered, so nbr can
         // only be in the row through an earlier update of the edge, and that
         // one would have marked the row edited.
         from = s + len;
@@ -472,20 +507,7 @@ __device__ __forceinline__ int grp_add_slot(const Lanes<W>& L, const Dev& g, uin
             continue;
         }
         if (!hit) {
-            if (L.leader() && (g.abl & ABL_NO_OVERFLOW)) {  // the ablation drops the edge
-                g.gctl[graph_of(g, x)].dropped = 1u;
-                flag_asym(g, x);
-            } else if (L.leader()) {
-                const uint32_t pos = atomicAdd(g.ovf_count, 1u);
-                if (pos < OVF_CAP) {
-                    g.ovf[pos].local_vertex_idx = x;
-                    g.ovf[pos].neighbor_global = nbr;
-                } else {
-                    atomicAdd(g.ovf_lost, 1ull);
-                    g.gctl[graph_of(g, x)].dropped = 1u;
-                }
-                flag_asym(g, x);
-            }
+            if (L.leader()) append_overflow(g, x, nbr);
             L.sync();
             return ADD_OVERFLOW;
         }
@@ -504,20 +526,19 @@ __device__ __forceinline__ int grp_add_slot(const Lanes<W>& L, const Dev& g, uin
         from = p + 1;  // lost the slot to a concurrent insert: keep scanning after it
     }
 }
-__device__ __forceinline__ int warp_add_slot(const Dev& g, uint32_t x, uint32_t nbr, bool exact) {
-    return grp_add_slot(Lanes<32>(), g, x, nbr, exact);
+__device__ __forceinline__ int warp_add_slot(const Dev& g, uint32_t x, uint32_t nbr) {
+    return grp_add_slot(Lanes<32>(), g, x, nbr);
 }
 
 // remove_local_neighbor: first slot equal to nbr becomes INV (lazy delete).
 // Returns whether an entry was removed.
 template <int W>
-__device__ __forceinline__ bool grp_remove_slot(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr,
-                                                bool exact) {
+__device__ __forceinline__ bool grp_remove_slot(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr) {
     const uint64_t s = g.rp[x];
-    const uint32_t bl = (!exact && g.blen) ? ld_cg(g.blen + x) : 0u;
+    const uint32_t bl = g.blen ? ld_cg(g.blen + x) : 0u;
     const uint64_t e = live_end(g, x, s);
     uint64_t from = s;
-    if (!exact && g.blen) {
+    if (g.blen) {
         if (bl && grp_run_remove(L, g, x, nbr, s, bl)) return true;
         from = s + bl;  // not live in the run: the tail
     } else if (pristine(g, x)) {
@@ -526,16 +547,10 @@ __device__ __forceinline__ bool grp_remove_slot(const Lanes<W>& L, const Dev& g,
             uint32_t old = 0;
             if (L.leader()) {
                 old = atomicCAS(g.col + p, nbr, INV);
-                if (old == nbr) {
-                    mark_dirty(g, x);
-                    if (g.live) atomicSub(g.live + x, 1u);
-                    if (g.blen) g.blen[x] = 0;  // an INV inside the run ends it
-                }
+                if (old == nbr) mark_dirty(g, x);
             }
             old = L.shfl(old, 0);
             if (old == nbr) return true;
-        } else if (exact) {
-            return false;  // absent from the sorted run and nothing after it
         }
     }
     for (;;) {
@@ -556,8 +571,8 @@ __device__ __forceinline__ bool grp_remove_slot(const Lanes<W>& L, const Dev& g,
         from = p + 1;
     }
 }
-__device__ __forceinline__ bool warp_remove_slot(const Dev& g, uint32_t x, uint32_t nbr, bool exact) {
-    return grp_remove_slot(Lanes<32>(), g, x, nbr, exact);
+__device__ __forceinline__ bool warp_remove_slot(const Dev& g, uint32_t x, uint32_t nbr) {
+    return grp_remove_slot(Lanes<32>(), g, x, nbr);
 }
 
 // ---------------- color selection (color_select.cuh:10-115) ----------------
@@ -574,6 +589,7 @@ __device__ __forceinline__ void add_color_bit(uint32_t c, uint32_t& lo, uint32_t
 
 // Histogram mode: first zero counter -> its color; else the first minimum.
 // Whole row (maxc counters) is loaded warp-wide, 16 bytes per lane per step.
+template <bool CA = false>
 __device__ __forceinline__ uint16_t warp_fac_hist(const uint32_t* h, uint32_t maxc) {
     const uint32_t lane = lane_id();
     uint32_t best_v = FULL, best_i = FULL;  // lane-local first minimum
@@ -581,7 +597,7 @@ __device__ __forceinline__ uint16_t warp_fac_hist(const uint32_t* h, uint32_t ma
         const uint32_t i = base + 4 * lane;
         uint4 q = make_uint4(FULL, FULL, FULL, FULL);
         const bool ok = i < maxc;
-        if (ok) q = ld_cg4(h + i);
+        if (ok) q = ld_w4<CA>(h + i);
         uint32_t zm = 0;
         if (ok) zm = (q.x == 0 ? 1u : 0u) | (q.y == 0 ? 2u : 0u) | (q.z == 0 ? 4u : 0u) | (q.w == 0 ? 8u : 0u);
         const uint32_t bz = __ballot_sync(FULL, zm != 0);
@@ -608,10 +624,11 @@ __device__ __forceinline__ uint16_t warp_fac_hist(const uint32_t* h, uint32_t ma
 
 // Bitmap mode fallback when all 64 bits are set: first color in 1..255 no live
 // neighbor holds (reading neighbor colors from `cols`), else 256.
+template <bool CA = false>
 __device__ __forceinline__ uint16_t warp_fac_scan(const Dev& g, uint32_t x, const uint32_t* cols) {
-    const uint64_t s = g.rp[x], e = live_end(g, x, s);
+    const uint64_t s = g.rp[x], e = live_end<CA>(g, x, s);
     uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    warp_gather_each<false>(g.col, s, e, g.n, cols, [&](uint32_t, uint32_t sw) {
+    warp_gather_each<false, 4, CA>(g.col, s, e, g.n, cols, [&](uint32_t, uint32_t sw) {
         const uint16_t c = color_of(sw);
         if (c > 0 && c < 256) {
 #pragma unroll
@@ -633,6 +650,7 @@ __device__ __forceinline__ uint16_t warp_fac_scan(const Dev& g, uint32_t x, cons
 // Colors 1..64 collect in a 64-bit lane mask, higher ones (up to 2047) in a
 // 2048-bit set the warp fills in shared memory while it scans the row (the
 // calling kernels run at most 8 warps per block).
+template <bool CA = false>
 __device__ __forceinline__ uint16_t warp_fac_exact(const Dev& g, uint32_t x, const uint32_t* cols) {
     __shared__ uint32_t s_used[8][64];
     uint32_t* used = s_used[(threadIdx.x >> 5) & 7];
@@ -641,8 +659,8 @@ __device__ __forceinline__ uint16_t warp_fac_exact(const Dev& g, uint32_t x, con
     used[lane + 32] = 0;
     __syncwarp();
     uint32_t lo = 0, hi = 0;
-    const uint64_t s = g.rp[x], e = live_end(g, x, s);
-    warp_gather_each<false>(g.col, s, e, g.n, cols, [&](uint32_t, uint32_t sw) {
+    const uint64_t s = g.rp[x], e = live_end<CA>(g, x, s);
+    warp_gather_each<false, 4, CA>(g.col, s, e, g.n, cols, [&](uint32_t, uint32_t sw) {
         const uint16_t c = color_of(sw);
         add_color_bit(c, lo, hi);
         if (c > 64 && c < 2048) atomicOr(&used[c >> 5], 1u << (c & 31));
@@ -670,13 +688,14 @@ __device__ __forceinline__ uint16_t warp_fac_exact(const Dev& g, uint32_t x, con
 }
 
 // FindAvailableColor: histogram row when the vertex has one, else bitmap.
+template <bool CA = false>
 __device__ __forceinline__ uint16_t warp_fac(const Dev& g, uint32_t x, const uint32_t* cols) {
     const uint32_t hd = __ldg(g.hdmap + x);
     if (hd != EMPTY && !(g.abl & ABL_FORCE_BITMAP))
-        return g.exact ? warp_fac_exact(g, x, cols) : warp_fac_hist(g.hist + (uint64_t)hd * g.maxc, g.maxc);
-    const uint64_t bmv = ld_cg(g.bm + x);
+        return g.exact ? warp_fac_exact<CA>(g, x, cols) : warp_fac_hist<CA>(g.hist + (uint64_t)hd * g.maxc, g.maxc);
+    const uint64_t bmv = ld_w<CA>(g.bm + x);
     if (~bmv) return (uint16_t)__ffsll((long long)~bmv);
-    return warp_fac_scan(g, x, cols);
+    return warp_fac_scan<CA>(g, x, cols);
 }
 
 // ---------------- incremental bitmap / histogram (color_select.cuh:120-209) ----------------
@@ -686,15 +705,16 @@ __device__ __forceinline__ uint16_t warp_fac(const Dev& g, uint32_t x, const uin
 // apply): the recolor walk sets one bit in every neighbor's bitmap, most of
 // them already set. Otherwise a fire-and-forget reduction: one vertex on the
 // update path, where the warp should not wait.
-template <bool READ_FIRST>
+template <bool READ_FIRST, bool CA = false>
 __device__ __forceinline__ void set_bm_bit(const Dev& g, uint32_t x, uint16_t c) {
     const unsigned long long bit = 1ull << (c - 1);
-    if (!READ_FIRST || !(ld_cg(g.bm + x) & bit)) atomicOr((unsigned long long*)(g.bm + x), bit);
+    if (!READ_FIRST || !(ld_w<CA>(g.bm + x) & bit)) atomicOr((unsigned long long*)(g.bm + x), bit);
 }
 
+template <bool CA = false>
 __device__ __forceinline__ void nbr_color_change(const Dev& g, uint32_t x, uint16_t oldc, uint16_t newc) {
     if (oldc == newc) return;
-    if (newc != 0 && newc <= 64) set_bm_bit<true>(g, x, newc);
+    if (newc != 0 && newc <= 64) set_bm_bit<true, CA>(g, x, newc);
     if (g.exact) return;  // no histogram rows
     const uint32_t hd = __ldg(g.hdmap + x);
     if (hd != EMPTY) {
@@ -806,19 +826,17 @@ __device__ __forceinline__ void warp_load_states2(const Dev& g, uint32_t u, uint
     sv = __shfl_sync(FULL, w, 1);
 }
 
-// try_color_reduction: after a delete freed `freed`, move to a lower color if one is open.
-// `stream_order` false (a concurrent batch) with exact selection on a row above
-// the threshold: instead of the full first-free scan, x moves to `freed` when no
+// try_color_reduction in a concurrent batch: after a delete freed `freed`, move
+// to a lower color if one is open. With exact selection on a row above the
+// threshold, instead of the full first-free scan, x moves to `freed` when no
 // live neighbor holds it any more (an early-exit scan; the full scan of a
-// high-degree row would almost always confirm the current color).
-// `state` is x's state word as the caller last read it (in stream order
-// nothing else changes it before this call; concurrently, a recolor re-reads it).
-__device__ __forceinline__ void warp_try_reduce(const Dev& g, uint32_t x, uint16_t freed, bool stream_order,
-                                                uint32_t state) {
+// high-degree row would almost always confirm the current color). `state` is
+// x's state word as the caller last read it (a recolor re-reads it).
+__device__ __forceinline__ void warp_try_reduce(const Dev& g, uint32_t x, uint16_t freed, uint32_t state) {
     const uint16_t cur = color_of(state);
     if (cur == 0) return;
     if (freed >= cur) return;
-    if (!stream_order && g.exact && __ldg(g.hdmap + x) != EMPTY) {
+    if (g.exact && __ldg(g.hdmap + x) != EMPTY) {
         if (freed == 0) return;
         if (g.hub_ops && row_len(g, x) > kHubRow) {
             // a holder is usually among the first neighbors; a hub row without
@@ -856,12 +874,9 @@ __device__ __forceinline__ uint32_t warp_color_uncolored(const Dev& g, uint32_t 
     return __shfl_sync(FULL, got, 0);
 }
 
-// ---------------- one update (local_update.cu:61-147) ----------------
+// ---------------- one update of a concurrent batch (local_update.cu:61-147) ----------------
 
-// `exact`: the caller is the only warp touching the graph (stream order), so a
-// pristine row's binary-search answer is final; concurrent callers fall back
-// to the linear scan whenever the search does not find the key.
-__device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v, uint8_t type, bool exact) {
+__device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v, uint8_t type) {
     if (g.touched && lane_id() == 0 && (type == SGC_UPDATE_ADD || type == SGC_UPDATE_DEL)) {
         // bitmap-class rows are revisited (their bitmaps rebuilt); a row with a
         // histogram class takes exact colors from its live neighbors instead,
@@ -869,29 +884,25 @@ __device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v,
         if (__ldg(g.hdmap + u) == EMPTY) mark_touched(g, u);
         if (__ldg(g.hdmap + v) == EMPTY) mark_touched(g, v);
     }
-    // The state words are read once, after the row edits, and kept: in stream
-    // order only this warp changes them, so the reference's re-reads give the
-    // same values; in a concurrent batch a later change by another warp is a
-    // color change (marked) or leaves this ADD's endpoints equal (caught by
-    // the check after the batch).
-    // In a concurrent batch the two row edits of an edge (u != v) touch two
-    // different rows and no other warp edits those slots of theirs, so the
-    // two halves of the warp make them at once (lanes 0-15 row u, 16-31 row
-    // v). In stream order they stay in order: the overflow buffer records
-    // u's entry before v's, as the reference does.
-    const bool halves = !exact && u != v;
+    // The state words are read once, after the row edits, and kept: a later
+    // change by another warp is a color change (marked) or leaves this ADD's
+    // endpoints equal (caught by the check after the batch).
+    // The two row edits of an edge (u != v) touch two different rows and no
+    // other warp edits those slots of theirs, so the two halves of the warp
+    // make them at once (lanes 0-15 row u, 16-31 row v).
+    const bool halves = u != v;
     if (type == SGC_UPDATE_ADD) {
         int ru, rv;
         if (halves) {
             const Lanes<16> H;
             const uint32_t x = H.base ? v : u, y = H.base ? u : v;  // one call site: the halves stay converged
-            const int r = grp_add_slot(H, g, x, y, false);
+            const int r = grp_add_slot(H, g, x, y);
             __syncwarp();
             ru = __shfl_sync(FULL, r, 0);
             rv = __shfl_sync(FULL, r, 16);
         } else {
-            ru = warp_add_slot(g, u, v, exact);
-            rv = warp_add_slot(g, v, u, exact);
+            ru = warp_add_slot(g, u, v);
+            rv = warp_add_slot(g, v, u);
         }
         if (ru != rv && lane_id() == 0) flag_asym(g, u);
         uint32_t su, sv;
@@ -911,10 +922,9 @@ __device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v,
         const uint16_t cu = color_of(su), cv = color_of(sv);
         if (cu == cv && cu != 0) {
             const uint32_t loser = prio_less(__ldg(g.deg + u), u, __ldg(g.deg + v), v) ? u : v;
-            // concurrent batches: a long histogram-class row's selection and
-            // walk go to the pass after the batch
-            const bool defer = !exact && g.hub_ops && __ldg(g.hdmap + loser) != EMPTY &&
-                               row_len(g, loser) > kHubRow && warp_defer(g, loser, HUB_RECOLOR, 0);
+            // a long histogram-class row's selection and walk go to the pass after the batch
+            const bool defer = g.hub_ops && __ldg(g.hdmap + loser) != EMPTY && row_len(g, loser) > kHubRow &&
+                               warp_defer(g, loser, HUB_RECOLOR, 0);
             if (!defer) warp_recolor(g, loser);
         }
     } else if (type == SGC_UPDATE_DEL) {
@@ -926,13 +936,13 @@ __device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v,
         if (halves) {
             const Lanes<16> H;
             const uint32_t x = H.base ? v : u, y = H.base ? u : v;
-            const int d = grp_remove_slot(H, g, x, y, false) ? 1 : 0;
+            const int d = grp_remove_slot(H, g, x, y) ? 1 : 0;
             __syncwarp();
             du = __shfl_sync(FULL, d, 0) != 0;
             dv = __shfl_sync(FULL, d, 16) != 0;
         } else {
-            du = warp_remove_slot(g, u, v, exact);
-            dv = warp_remove_slot(g, v, u, exact);
+            du = warp_remove_slot(g, u, v);
+            dv = warp_remove_slot(g, v, u);
         }
         if (lane_id() == 0) {
             if (du != dv) flag_asym(g, u);
@@ -940,9 +950,281 @@ __device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v,
             removed_nbr(g, v, fv);
         }
         __syncwarp();
-        warp_try_reduce(g, u, fu, exact, su);
+        warp_try_reduce(g, u, fu, su);
         if (v == u) sv = warp_load_state(g, v);
-        warp_try_reduce(g, v, fv, exact, sv);
+        warp_try_reduce(g, v, fv, sv);
+    }
+}
+
+// ---------------- updates in stream order (local_update.cu:61-147) ----------------
+//
+// One warp of a block applies updates one after another; nothing else changes
+// the graph meanwhile, so no word needs an atomic whose result is waited for,
+// and every word may sit in the SM's L1. What bounds it is the chain of
+// dependent loads and instructions per update, so the block's other warps
+// prepare updates ahead of the one applying (seq_prepare): they search both
+// rows and leave the slots in shared memory, and the lines they read in L1.
+// A row edited after it was searched is settled again from the slots edited
+// since (seq_settle), which the applying warp logs.
+
+constexpr uint32_t kSeqWarps = 16;  // one applies, fifteen prepare
+constexpr uint32_t kSeqChunk = kSeqWarps - 1;  // updates between two block barriers: one per preparing warp
+constexpr uint32_t kSeqMarks = 2048;
+
+// Where the edit of a neighbor lands: the slot holding it (SEQ_HIT), for an
+// ADD else the first free one (SEQ_FREE), else none.
+enum : uint32_t { SEQ_FREE = ADD_INSERTED, SEQ_HIT = ADD_PRESENT, SEQ_NONE = ADD_OVERFLOW };
+
+// One endpoint of one update as it was prepared.
+struct alignas(16) SeqEnd {
+    uint64_t s;    // row start
+    uint32_t q;    // the edit's slot, relative to s
+    uint32_t r;    // SEQ_*
+    uint32_t hw, bl, hd;
+    uint32_t ed;   // the row was edited before (the bit is only ever set)
+};
+
+// Shared memory of a block that applies in stream order.
+struct SeqShared {
+    SeqEnd end[2][kSeqChunk][2];  // by chunk parity, update, endpoint
+    uint4 rec[2][kSeqChunk];
+    uint2 log[2][2 * kSeqChunk];  // {row, slot} of every edit of the current and the previous chunk
+    uint32_t mark[kSeqMarks];     // by hashed row: the last chunk that edited one
+    uint32_t sink[32 * kSeqWarps];
+};
+
+// Half-warp: where the edit of y lands in row x ([s, cap), mark hw). The first
+// free slot lies at or below the mark. A row that was never edited is sorted
+// without holes: a longer one is searched.
+__device__ __forceinline__ void seq_locate(const Lanes<16>& H, const Dev& g, uint32_t y, uint64_t cap, bool add,
+                                           SeqEnd& d) {
+    uint64_t e = d.s + d.hw, p = 0;
+    if (e > cap) {
+        if (H.leader()) atomicOr(g.err, ERR_ROW);
+        e = cap;
+    }
+    if (e - d.s > 64 && !d.ed) {
+        p = grp_bsearch<true>(H, g.col, d.s, e, y);
+        d.r = p != ~0ull ? SEQ_HIT : (add && e < cap ? SEQ_FREE : SEQ_NONE);
+        if (p == ~0ull) p = e;
+    } else {
+        const uint64_t lim = add && e < cap ? e + 1 : e;
+        uint32_t v = 0;
+        const bool hit =
+            grp_find<true>(H, g.col, d.s, lim, [y, add](uint32_t t) { return t == y || (add && t == INV); }, p, v);
+        d.r = !hit ? SEQ_NONE : (v == y ? SEQ_HIT : SEQ_FREE);
+    }
+    d.q = (uint32_t)(p - d.s);
+}
+
+__device__ __forceinline__ void seq_read(const Dev& g, uint32_t x, SeqEnd& d) {
+    d.hw = ld_w<true>(g.hw + x);
+    d.ed = (ld_w<true>(g.edited + (x >> 5)) >> (x & 31)) & 1u;
+    d.bl = g.blen ? ld_w<true>(g.blen + x) : 0u;
+}
+
+// A preparing warp: both endpoints of one update, a half-warp each.
+__device__ __forceinline__ void seq_prepare(const Dev& g, SeqShared& sh, uint32_t par, uint32_t j, const uint4& r) {
+    if (lane_id() == 0) sh.rec[par][j] = r;
+    if (r.x >= g.n || r.y >= g.n) return;
+    const Lanes<16> H;
+    const uint32_t x = H.base ? r.y : r.x, y = H.base ? r.x : r.y;
+    SeqEnd d;
+    d.s = g.rp[x];
+    const uint64_t cap = g.rp[x + 1];
+    seq_read(g, x, d);
+    d.hd = __ldg(g.hdmap + x);
+    uint32_t sink = ld_w<true>(g.st + x) ^ (uint32_t)ld_w<true>(g.bm + x);
+    seq_locate(H, g, y, cap, (r.z & 0xFFu) == SGC_UPDATE_ADD, d);
+    if (H.leader()) sh.end[par][j][H.base >> 4] = d;
+    if (d.hd != EMPTY && !g.exact) {  // the counters a selection reads first
+        const uint32_t* h = g.hist + (uint64_t)d.hd * g.maxc;
+        for (uint32_t i = 4 * H.lane; i < g.maxc && i < 128; i += 64) sink ^= ld_w4<true>(h + i).x;
+    }
+    sh.sink[threadIdx.x] = sink;  // those loads are made for the lines they leave in L1
+    __syncwarp();
+}
+
+// Half-warp: row x may have been edited since `d` was prepared, or while it was
+// (the search then saw some of those edits, in any order). Every slot edited
+// since is in the log; no other slot changed. So the edit lands at the first of
+// the prepared slot (unless it is logged), the logged slots that match now, and,
+// when the search ran into the free slots past the mark, the present mark. A
+// logged slot that no longer matches, with no match before it, leaves the rest
+// of the row unknown, and a row first edited meanwhile may have misled the
+// sorted search: both are searched again.
+__device__ __forceinline__ void seq_settle(const Lanes<16>& H, const Dev& g, const SeqShared& sh, uint32_t x,
+                                           uint32_t y, bool add, SeqEnd& d) {
+    const uint64_t cap = g.rp[x + 1];
+    const bool sorted = !d.ed, tail = add && (d.r == SEQ_NONE || (d.r == SEQ_FREE && d.q == d.hw));
+    seq_read(g, x, d);
+    uint32_t first = NOSLOT, val = 0;  // the first logged slot that matches now
+    bool logged = false;
+    for (uint32_t k = H.lane; k < 4 * kSeqChunk; k += 16) {
+        const uint2 e = (&sh.log[0][0])[k];
+        if (e.x != x) continue;
+        logged |= e.y == d.q;
+        const uint32_t t = ld_w<true>(g.col + d.s + e.y);
+        if ((t == y || (add && t == INV)) && e.y < first) {
+            first = e.y;
+            val = t;
+        }
+    }
+    logged = d.r != SEQ_NONE && H.ballot(logged) != 0;
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) {
+        const uint32_t o = __shfl_xor_sync(H.mask, first, off), ov = __shfl_xor_sync(H.mask, val, off);
+        if (o < first) {
+            first = o;
+            val = ov;
+        }
+    }
+    if (tail) {
+        d.r = d.s + d.hw < cap ? SEQ_FREE : SEQ_NONE;
+        d.q = d.hw;
+        logged = false;
+    }
+    if (sorted) {
+        seq_locate(H, g, y, cap, add, d);
+    } else if (first != NOSLOT && (d.r == SEQ_NONE || first <= d.q)) {
+        d.q = first;
+        d.r = val == y ? SEQ_HIT : SEQ_FREE;
+    } else if (logged) {
+        seq_locate(H, g, y, cap, add, d);
+    }
+}
+
+// One leader lane per edited row: the slot, the row's bookkeeping and the log.
+__device__ __forceinline__ void seq_edit(const Dev& g, SeqShared& sh, uint32_t chunk, uint2* log, uint32_t x,
+                                         uint32_t y, const SeqEnd& d, bool add, bool act) {
+    *log = make_uint2(act ? x : NOSLOT, d.q);
+    if (!act) return;
+    sh.mark[x % kSeqMarks] = chunk;
+    g.col[d.s + d.q] = add ? y : INV;
+    if (add && d.q >= d.hw) g.hw[x] = d.q + 1;
+    if (g.live) atomicAdd(g.live + x, add ? 1u : ~0u);
+    if (!add && d.q < d.bl) g.blen[x] = 0;  // an INV inside the run ends it
+    atomicOr(g.dirty + (x >> 5), 1u << (x & 31));
+    if (!d.ed) atomicOr(g.edited + (x >> 5), 1u << (x & 31));
+}
+
+// Adds `by` to one histogram counter (one lane; `shared`: another lane adds to the same row).
+__device__ __forceinline__ void seq_count(uint32_t* h, uint32_t by, bool shared) {
+    if (shared) atomicAdd(h, by);
+    else *h = ld_w<true>(h) + by;
+}
+
+// recolor_vertex on x, read as state word `cur`: to `newc`, when that is another
+// color; the change is walked to every live neighbor.
+__device__ __forceinline__ void seq_recolor(const Dev& g, uint32_t x, uint16_t newc, uint32_t cur) {
+    const uint16_t oldc = color_of(cur);
+    if (newc == oldc) return;
+    if (lane_id() == 0) {
+        g.st[x] = pack(newc, (uint16_t)(version_of(cur) + 1));
+        mark_touched(g, x);
+        note_color(g, x);
+    }
+    const uint64_t s = g.rp[x], e = live_end<true>(g, x, s);
+    warp_for_each<true>(g.col, s, e, [&](uint64_t, uint32_t ng) {
+        if (ng == INV || ng >= g.n) return;
+        nbr_color_change<true>(g, ng, oldc, newc);
+    });
+    __syncwarp();
+}
+
+__device__ __forceinline__ uint32_t seq_color_uncolored(const Dev& g, uint32_t x) {
+    const uint32_t w = pack(warp_fac<true>(g, x, g.st), 1);
+    if (lane_id() == 0) {
+        g.st[x] = w;
+        mark_touched(g, x);
+        note_color(g, x);
+    }
+    __syncwarp();
+    return w;
+}
+
+__device__ __forceinline__ void seq_try_reduce(const Dev& g, uint32_t x, uint16_t freed, uint32_t state) {
+    const uint16_t cur = color_of(state);
+    if (cur == 0 || freed >= cur) return;
+    const uint16_t best = warp_fac<true>(g, x, g.st);
+    if (best < cur) seq_recolor(g, x, best, state);
+}
+
+// The applying warp: update j of the chunk `chunk` (its parity: the buffers).
+__device__ __forceinline__ void seq_apply(const Dev& g, SeqShared& sh, uint32_t chunk, uint32_t j) {
+    const uint32_t par = chunk & 1u;
+    const uint4 rec = sh.rec[par][j];
+    const uint32_t u = rec.x, v = rec.y;
+    const Lanes<16> H;
+    uint2* log = &sh.log[par][2 * j + (H.base >> 4)];
+    const uint32_t type = rec.z & 0xFFu;
+    if (u >= g.n || v >= g.n || (type != SGC_UPDATE_ADD && type != SGC_UPDATE_DEL)) {
+        if (H.leader()) *log = make_uint2(NOSLOT, 0);
+        if ((u >= g.n || v >= g.n) && lane_id() == 0) atomicAdd(g.nskip, 1ull);  // get_owned_index miss: skipped
+        return;
+    }
+    const bool add = type == SGC_UPDATE_ADD;
+    const uint32_t x = H.base ? v : u, y = H.base ? u : v;
+    const uint32_t stw = ld_w<true>(g.st + x);
+    uint64_t bmw = ld_w<true>(g.bm + x);
+    SeqEnd d = sh.end[par][j][H.base >> 4];
+    const bool stale = sh.mark[x % kSeqMarks] + 1 >= chunk;  // edited in this chunk or the one before
+    if (d.hd == EMPTY && H.leader()) mark_touched(g, x);     // as in warp_apply
+    if (stale) seq_settle(H, g, sh, x, y, add, d);
+    __syncwarp();
+    const uint32_t want = add ? SEQ_FREE : SEQ_HIT;
+    if (u != v) {
+        if (H.leader()) seq_edit(g, sh, chunk, log, x, y, d, add, d.r == want);
+    } else {  // one row, edited twice: the second edit sees the first
+        if (lane_id() == 0) seq_edit(g, sh, chunk, log, x, y, d, add, d.r == want);
+        __syncwarp();
+        if (H.base) {
+            seq_read(g, x, d);
+            seq_locate(H, g, y, g.rp[x + 1], add, d);
+            if (H.leader()) seq_edit(g, sh, chunk, log, x, y, d, add, d.r == want);
+        }
+    }
+    __syncwarp();
+    const uint32_t ru = __shfl_sync(FULL, d.r, 0), rv = __shfl_sync(FULL, d.r, 16);
+    if (lane_id() == 0 && (ru != rv || ru == SEQ_NONE)) {
+        if (add && ru == SEQ_NONE) append_overflow(g, u, v);  // u's entry before v's
+        if (add && rv == SEQ_NONE) append_overflow(g, v, u);
+        if (ru != rv) flag_asym(g, u);
+    }
+    uint32_t su = __shfl_sync(FULL, stw, 0), sv = __shfl_sync(FULL, stw, 16);
+    if (add) {
+        if (color_of(su) == 0 || color_of(sv) == 0) {
+            if (color_of(su) == 0) {
+                su = seq_color_uncolored(g, u);
+                if (v == u) sv = su;
+            }
+            if (color_of(sv) == 0) {
+                if (lane_id() == 0) new_nbr(g, v, color_of(su));
+                __syncwarp();
+                sv = seq_color_uncolored(g, v);
+            }
+            bmw = ld_w<true>(g.bm + x);
+        }
+        const uint16_t cu = color_of(su), cv = color_of(sv), oc = H.base ? cu : cv;
+        if (H.leader() && oc != 0) {  // new_nbr
+            const uint64_t bit = oc <= 64 ? 1ull << (oc - 1) : 0ull;
+            if (bit & ~bmw) g.bm[x] = bmw | bit;
+            if (d.hd != EMPTY && !g.exact && oc <= g.maxc) seq_count(g.hist + (uint64_t)d.hd * g.maxc + oc - 1, 1u, u == v);
+        }
+        __syncwarp();
+        if (cu == cv && cu != 0) {
+            const bool first = prio_less(__ldg(g.deg + u), u, __ldg(g.deg + v), v);
+            const uint32_t loser = first ? u : v;
+            seq_recolor(g, loser, warp_fac<true>(g, loser, g.st), first ? su : sv);
+        }
+    } else {
+        const uint16_t fu = color_of(sv), fv = color_of(su), fx = H.base ? fv : fu;
+        if (H.leader() && fx != 0 && d.hd != EMPTY && !g.exact && fx <= g.maxc)  // removed_nbr
+            seq_count(g.hist + (uint64_t)d.hd * g.maxc + fx - 1, ~0u, u == v);
+        __syncwarp();
+        seq_try_reduce(g, u, fu, su);
+        if (v == u) sv = ld_w<true>(g.st + v);
+        seq_try_reduce(g, v, fv, sv);
     }
 }
 
