@@ -43,10 +43,11 @@ typedef struct sgc_handle sgc_handle;
  * never rebuilt and drift, color_select.cuh:120-209). No histogram rows are
  * allocated. Bit-exact parity with the reference needs this flag off. */
 #define SGC_OPT_EXACT_SELECT 2u
-/* With SGC_OPT_EXACT_SELECT, a publish after concurrent batches replays one
- * captured CUDA graph (compaction, drain, the repair loop as a conditional
- * while-node, snapshot): one host synchronization per epoch instead of one per
- * sweep. Sweeps are not timed one by one (sgc_stats.sweep_ms stays 0). */
+/* On handles with SGC_OPT_PROFILE a repair runs each sweep's passes as kernels
+ * of their own and times them, a host synchronization per sweep. With
+ * SGC_OPT_EXACT_SELECT this flag keeps a publish after concurrent batches to the
+ * one kernel that runs the whole loop otherwise, one host synchronization per
+ * epoch: those sweeps are not timed (sgc_stats.sweep_ms stays 0). */
 #define SGC_OPT_GRAPH_PUBLISH 4u
 /* With SGC_OPT_EXACT_SELECT, compaction also sorts every row of at most 1024
  * live entries into one base run, and compacts a row whose unsorted tail (the

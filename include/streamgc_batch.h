@@ -13,7 +13,7 @@
  *     one persistent launch fed by a device work queue, repairs, and publishes
  *     a snapshot for each graph whose epoch closed;
  *   - the tick runs as a captured CUDA graph (its repair loop is a
- *     conditional while-node), so a tick costs one launch from the host;
+ *     one kernel, long sweeps in a while-node), so a tick costs one launch from the host;
  *   - per graph, the repair state (clean / mirror-complete / forced) is kept
  *     apart, so with SGC_BATCH_STREAM_ORDER a graph's colors do not depend on
  *     the other graphs in the batch.

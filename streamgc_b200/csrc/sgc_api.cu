@@ -149,50 +149,63 @@ void publish_snapshot(sgc_handle* h) {
 //   vertices touched by updates since the last repair -- when that repair ended
 //   proper, the rows are mirror-complete and `force_full` is off: every new
 //   conflict then has an endpoint among the touched vertices.
-int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full) {
+//   `timed`: each sweep's passes as kernels of their own with events between
+//   them (SGC_OPT_PROFILE); otherwise the loop runs in one cooperative kernel
+//   except for sweeps over many vertices.
+int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool timed) {
     const bool indep = h->g.exact != 0;
     const SweepMode mode = indep ? SWEEP_INDEP : SWEEP_TIER1;
     const uint32_t every = h->opt.full_repair_every;
     if (every && h->repairs_since_full + 1 >= every) force_full = true;
-    RepairCtl* hin = h->h_rc_in;
-    hin->mode = (uint32_t)mode;
-    hin->max_sweeps = indep ? 64u : 20u;
-    hin->force_all = force_full ? 1u : 0u;
-    CK(cudaMemcpyAsync(h->sb.rc, hin, 12, cudaMemcpyHostToDevice, h->stream));
-    const size_t mwords = ((h->n + 31) / 32) * 4;
-    CK(cudaMemsetAsync(h->sb.wmark, 0, mwords, h->stream));
-    CK(cudaMemsetAsync(h->sb.rbits, 0, mwords, h->stream));
-    CK(cudaMemsetAsync(h->sb.needf, 0, h->n, h->stream));  // no vertex starts conflicted
-    launch_repair_begin(h->g, h->sb, mode, h->num_sms, h->stream);
-    h->launches += (mode == SWEEP_INDEP && h->g.touched) ? 2 : 1;
-    const bool prof = (h->opt.flags & SGC_OPT_PROFILE) != 0;
+    const RepairIn in{(uint32_t)mode, indep ? 64u : 20u, force_full ? 1u : 0u};
+    timed = timed && (h->opt.flags & SGC_OPT_PROFILE);
     RepairCtl* rc = h->h_rc_out;
-    for (uint32_t sweeps = 0;; sweeps++) {
-        if (sweeps > hin->max_sweeps) return fail(SGC_EDEVICE, "repair loop ran past %u sweeps", hin->max_sweeps);
+    auto read_back = [&]() -> int {
+        CK(cudaMemcpyAsync(rc, h->sb.rc, sizeof(RepairCtl), cudaMemcpyDeviceToHost, h->stream));
+        h->d2h_bytes += sizeof(RepairCtl);
+        return sync(h);
+    };
+    if (timed) {
+        RepairCtl* hin = h->h_rc_in;
+        hin->mode = in.mode;
+        hin->max_sweeps = in.max_sweeps;
+        hin->force_all = in.force_all;
+        CK(cudaMemcpyAsync(h->sb.rc, hin, 12, cudaMemcpyHostToDevice, h->stream));
+        const size_t mwords = ((h->n + 31) / 32) * 4;
+        CK(cudaMemsetAsync(h->sb.wmark, 0, mwords, h->stream));
+        CK(cudaMemsetAsync(h->sb.rbits, 0, mwords, h->stream));
+        CK(cudaMemsetAsync(h->sb.needf, 0, h->n, h->stream));  // no vertex starts conflicted
+        launch_repair_begin(h->g, h->sb, mode, h->num_sms, h->stream);
+        h->launches += (mode == SWEEP_INDEP && h->g.touched) ? 2 : 1;
+    } else {
+        launch_repair_fused(h->g, h->sb, &in, h->num_sms, h->stream, nullptr);
+        h->launches += 1;
+        TRY(check_cuda("repair"));
+        TRY(read_back());
+    }
+    for (uint32_t sweeps = 0; timed || rc->cont; sweeps++) {
+        if (sweeps > in.max_sweeps) return fail(SGC_EDEVICE, "repair loop ran past %u sweeps", in.max_sweeps);
         sgc_handle::SweepEvents se{};
-        if (prof) {
+        if (timed) {
             for (int k = 0; k < 5; k++) se.ev[k] = take_event(h);
             cudaEventRecord(se.ev[0], h->stream);
         }
-        launch_repair_sweep(h->g, h->sb, mode, h->num_sms, h->stream, prof ? se.ev + 1 : nullptr);
-        if (prof) {
+        launch_repair_sweep(h->g, h->sb, mode, h->num_sms, h->stream, timed ? se.ev + 1 : nullptr);
+        if (timed) {
             cudaEventRecord(se.ev[4], h->stream);
             h->ev_pending.push_back(se);
         }
         launch_repair_step(h->g, h->sb, h->num_sms, h->stream, nullptr);
         h->launches += 1 + (mode == SWEEP_INDEP ? 6 : 4) + 3;
-        CK(cudaMemcpyAsync(rc, h->sb.rc, sizeof(RepairCtl), cudaMemcpyDeviceToHost, h->stream));
-        h->d2h_bytes += sizeof(RepairCtl);
-        TRY(sync(h));
+        if (!timed) {
+            launch_repair_fused(h->g, h->sb, nullptr, h->num_sms, h->stream, nullptr);
+            h->launches += 1;
+        }
+        TRY(read_back());
         if (!rc->cont) break;
     }
     TRY(check_cuda("repair"));
-    if (prof) {
-        unsigned long long sw[2];
-        CK(cudaMemcpyAsync(sw, h->sb.swept, 16, cudaMemcpyDeviceToHost, h->stream));
-        TRY(sync(h));
-        h->sweep_bytes += 8ull * sw[0] + 28ull * sw[1];
-    }
+    if (h->opt.flags & (SGC_OPT_PROFILE | SGC_OPT_GRAPH_PUBLISH)) h->sweep_bytes += 8ull * rc->swept[0] + 28ull * rc->swept[1];
     return finish_repair(h, rep);
 }
 
@@ -268,121 +281,6 @@ int ensure_ingest(sgc_handle* h) {
     return SGC_OK;
 }
 
-// ---- the concurrent configuration's publish as a CUDA graph ----
-//
-// compaction of edited rows, overflow drain, the repair's start, a
-// conditional while-node { sweep, step } and the snapshot into one half of
-// the double buffer, captured once per half; the repair's host fields (mode,
-// sweep cap, full repair) reach the device through the graph's first copy,
-// from pinned memory written before each launch. One host synchronization per
-// epoch instead of one per sweep.
-
-void enqueue_publish_head(sgc_handle* h, cudaStream_t s) {
-    cudaMemsetAsync(&h->ctl->dirty_count, 0, 4, s);
-    launch_dirty_list(h->g, h->dirty_list, &h->ctl->dirty_count, s);
-    launch_compact(h->g, h->dirty_list, &h->ctl->dirty_count, h->n, false, s, (h->opt.flags & SGC_OPT_SORTED_ROWS) != 0);
-    launch_take_overflow(h->g, &h->ctl->drain_n, s);
-    launch_drain(h->g, &h->ctl->drain_n, false, &h->ctl->drain_failed, s);
-    cudaMemcpyAsync(h->sb.rc, h->h_rc_in, 12, cudaMemcpyHostToDevice, s);
-    const size_t mwords = ((h->n + 31) / 32) * 4;
-    cudaMemsetAsync(h->sb.wmark, 0, mwords, s);
-    cudaMemsetAsync(h->sb.rbits, 0, mwords, s);
-    cudaMemsetAsync(h->sb.needf, 0, h->n, s);
-    launch_repair_begin(h->g, h->sb, SWEEP_INDEP, h->num_sms, s);
-}
-
-void drop_publish_graphs(sgc_handle* h) {
-    for (int k = 0; k < 2; k++) {
-        if (h->pub_exec[k]) cudaGraphExecDestroy(h->pub_exec[k]);
-        if (h->pub_graph[k]) cudaGraphDestroy(h->pub_graph[k]);
-        h->pub_exec[k] = nullptr;
-        h->pub_graph[k] = nullptr;
-    }
-}
-
-int capture_publish_impl(sgc_handle* h, int back) {
-    cudaStream_t s = h->stream;
-    cudaGraph_t& graph = h->pub_graph[back];
-    CK(cudaGraphCreate(&graph, 0));
-    cudaGraphConditionalHandle cond;
-    CK(cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault));
-    CK(cudaStreamBeginCaptureToGraph(s, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    enqueue_publish_head(h, s);
-    cudaStreamCaptureStatus st;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    CK(cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &deps, &ndeps));
-    std::vector<cudaGraphNode_t> head_tail(deps, deps + ndeps);
-    cudaGraph_t g0 = nullptr;
-    CK(cudaStreamEndCapture(s, &g0));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = cond;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    CK(cudaGraphAddNode(&cnode, graph, head_tail.data(), head_tail.size(), &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    CK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    launch_repair_sweep(h->g, h->sb, SWEEP_INDEP, h->num_sms, s);
-    launch_repair_step(h->g, h->sb, h->num_sms, s, &cond);
-    cudaGraph_t g1 = nullptr;
-    CK(cudaStreamEndCapture(s, &g1));
-    CK(cudaStreamBeginCaptureToGraph(s, graph, &cnode, nullptr, 1, cudaStreamCaptureModeThreadLocal));
-    if (h->g.chg) launch_snapshot_changes(h->g, h->chg_prev, h->snap[back], s);
-    else launch_snapshot(h->g, h->snap[back], s);
-    cudaMemcpyAsync(h->h_rc_out, h->sb.rc, sizeof(RepairCtl), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(h->h_small + 32, h->sb.swept, 16, cudaMemcpyDeviceToHost, s);
-    cudaGraph_t g2 = nullptr;
-    CK(cudaStreamEndCapture(s, &g2));
-    CK(cudaGraphInstantiate(&h->pub_exec[back], graph, 0));
-    return SGC_OK;
-}
-
-int capture_publish(sgc_handle* h, int back) {
-    const int r = capture_publish_impl(h, back);
-    if (r != SGC_OK) {  // leave the stream out of capture mode; the eager publish takes over
-        cudaStreamCaptureStatus st;
-        if (cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone) {
-            cudaGraph_t g = nullptr;
-            cudaStreamEndCapture(h->stream, &g);
-            if (g) cudaGraphDestroy(g);
-        }
-        cudaGetLastError();
-        drop_publish_graphs(h);
-        h->pub_graph_failed = true;
-    }
-    return r;
-}
-
-int publish_graph(sgc_handle* h, sgc_repair_report* rep) {
-    const int back = 1 - h->front;
-    const uint32_t every = h->opt.full_repair_every;
-    RepairCtl* hin = h->h_rc_in;  // read by the graph's first copy
-    hin->mode = (uint32_t)SWEEP_INDEP;
-    hin->max_sweeps = 64u;
-    hin->force_all = (every && h->repairs_since_full + 1 >= every) ? 1u : 0u;
-    CK(cudaGraphLaunch(h->pub_exec[back], h->stream));
-    TRY(sync(h));
-    TRY(check_cuda("publish graph"));
-    const RepairCtl* rc = h->h_rc_out;
-    const unsigned long long* sw = (const unsigned long long*)(h->h_small + 32);
-    h->sweep_bytes += 8ull * sw[0] + 28ull * sw[1];
-    h->launches += (h->g.touched ? 6 : 5) + 10ull * rc->it + 1;
-    h->d2h_bytes += sizeof(RepairCtl) + 16;
-    sgc_repair_report r{};
-    TRY(finish_repair(h, &r));
-    if (r.tier2_ran || (h->g.chg && h->snap_full > 0)) {  // Tier-2 changed colors after the graph's
-        launch_snapshot(h->g, h->snap[back], h->stream);      // snapshot, or a full one is due: take it again
-        h->launches += 1;
-        if (h->snap_full > 0) h->snap_full--;
-    }
-    h->front = back;
-    h->epochs++;
-    if (rep) *rep = r;
-    return check_cuda("publish");
-}
-
 int read_drain(sgc_handle* h, sgc_repair_report* rep, unsigned long long before_failed) {
     CK(cudaMemcpyAsync(h->h_small, &h->ctl->drain_n, 4, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaMemcpyAsync(h->h_small + 2, &h->ctl->drain_failed, 8, cudaMemcpyDeviceToHost, h->stream));
@@ -419,7 +317,6 @@ int sgc_destroy(sgc_handle* h) {
     if (!h) return SGC_OK;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    drop_publish_graphs(h);
     if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
     for (int k = 0; k < 2; k++) {
         if (h->slot_host[k]) cudaFreeHost(h->slot_host[k]);
@@ -641,12 +538,14 @@ int sgci::create_internal(const StreamGCConfig* cfg, const sgc_options* opt_in, 
     A(&sb.wmark, (n + 31) / 32 + 1, 0);
     A(&sb.wl, n);
     A(&sb.wl_count, 4, 0);
+    sb.next_items = sb.wl_count + 1;
     A(&sb.swept, 2, 0);
     A(&sb.needf, n, 0);
     A(&sb.need_v, n);
     A(&sb.need_count, 4, 0);
     A(&sb.rbits, (n + 31) / 32 + 1, 0);
     A(&sb.rc, 1, 0);
+    A(&sb.bar, 1, 0);
     sb.tile = opt.repair_tile;
     sb.G = G;
     if (g.exact) A(&g.touched, (n + 31) / 32 + 1, 0);
@@ -882,7 +781,7 @@ int sgc_repair(sgc_handle* h, sgc_repair_report* rep) {
     TRY(drain(h, h->last_mode == SGC_MODE_DETERMINISTIC, &h->ctl->drain_failed));
     // drain_and_compact's rebuild is subsumed: the first (full) sweep rebuilds every bitmap first.
     TRY(read_drain(h, &r, before));
-    TRY(repair_loop(h, &r, true));
+    TRY(repair_loop(h, &r, true, true));
     if (rep) *rep = r;
     return SGC_OK;
 }
@@ -890,15 +789,12 @@ int sgc_repair(sgc_handle* h, sgc_repair_report* rep) {
 int sgc_publish(sgc_handle* h, sgc_repair_report* rep) {
     if (!h) return fail(SGC_EINVAL, "null handle");
     CK(cudaSetDevice(h->device));
-    if ((h->opt.flags & SGC_OPT_GRAPH_PUBLISH) && h->g.exact && h->last_mode == SGC_MODE_CONCURRENT &&
-        !h->pub_graph_failed) {
-        const int back = 1 - h->front;
-        if (h->pub_exec[back] || capture_publish(h, back) == SGC_OK) return publish_graph(h, rep);
-    }
+    // SGC_OPT_GRAPH_PUBLISH: sweeps are not timed one by one
+    const bool whole = (h->opt.flags & SGC_OPT_GRAPH_PUBLISH) && h->g.exact && h->last_mode == SGC_MODE_CONCURRENT;
     sgc_repair_report r{};
     TRY(compact_dirty(h, false));
     TRY(drain(h, h->last_mode == SGC_MODE_DETERMINISTIC, &h->ctl->drain_failed));
-    TRY(repair_loop(h, &r, false));
+    TRY(repair_loop(h, &r, false, !whole));
     publish_snapshot(h);
     h->epochs++;
     if (rep) *rep = r;

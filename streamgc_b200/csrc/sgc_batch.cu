@@ -9,7 +9,8 @@
 //   2. compacts edited rows and drains the overflow buffer;
 //   3. repairs with the independent-set rule, each graph starting from its
 //      touched vertices (or from all of them when its repair must be full);
-//      the loop is a conditional while-node of the captured CUDA graph;
+//      the loop is one kernel, its sweeps over many vertices a conditional
+//      while-node of the captured CUDA graph;
 //   4. publishes a snapshot for each graph whose epoch closed (double buffer
 //      per graph: queries read the other half while the tick writes);
 //   5. copies the loop state back for the host.
@@ -117,8 +118,9 @@ void drop_graph(sgc_batch* b) {
     b->graph = nullptr;
 }
 
-// Everything of a tick before the repair loop.
-void enqueue_head(sgc_batch* b, cudaStream_t s) {
+// A tick up to and with the repair (its sweeps over many vertices follow while
+// its control block says so; `cond` then holds that).
+void enqueue_head(sgc_batch* b, cudaStream_t s, const cudaGraphConditionalHandle* cond) {
     sgc_handle* h = b->h;
     if (b->flags & SGC_BATCH_STREAM_ORDER)
         launch_seg_apply(h->g, h->d_batch, b->d_segs, b->d_dyn, b->G, h->num_sms, s);
@@ -130,11 +132,8 @@ void enqueue_head(sgc_batch* b, cudaStream_t s) {
     launch_compact(h->g, h->dirty_list, &h->ctl->dirty_count, h->n, false, s, (h->opt.flags & SGC_OPT_SORTED_ROWS) != 0);
     launch_take_overflow(h->g, &h->ctl->drain_n, s);
     launch_drain(h->g, &h->ctl->drain_n, (b->flags & SGC_BATCH_STREAM_ORDER) != 0, &h->ctl->drain_failed, s);
-    const size_t mwords = ((h->n + 31) / 32) * 4;
-    cudaMemsetAsync(h->sb.wmark, 0, mwords, s);
-    cudaMemsetAsync(h->sb.rbits, 0, mwords, s);
-    cudaMemsetAsync(h->sb.needf, 0, h->n, s);
-    launch_repair_begin(h->g, h->sb, SWEEP_INDEP, h->num_sms, s);
+    const RepairIn in{(uint32_t)SWEEP_INDEP, 64u, 0u};
+    launch_repair_fused(h->g, h->sb, &in, h->num_sms, s, cond);
 }
 
 void enqueue_tail(sgc_batch* b, cudaStream_t s) {
@@ -143,7 +142,8 @@ void enqueue_tail(sgc_batch* b, cudaStream_t s) {
     cudaMemcpyAsync(h->h_rc_out, h->sb.rc, sizeof(RepairCtl), cudaMemcpyDeviceToHost, s);
 }
 
-// Captures the whole tick: head, while-node { sweep, step }, tail.
+// Captures the whole tick: head, while-node { sweep, step } for what the repair
+// left to it, tail.
 int capture_tick_impl(sgc_batch* b);
 int capture_tick(sgc_batch* b) {
     const int r = capture_tick_impl(b);
@@ -166,7 +166,7 @@ int capture_tick_impl(sgc_batch* b) {
     cudaGraphConditionalHandle cond;
     CK(cudaGraphConditionalHandleCreate(&cond, b->graph, 1, cudaGraphCondAssignDefault));
     CK(cudaStreamBeginCaptureToGraph(s, b->graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    enqueue_head(b, s);
+    enqueue_head(b, s, &cond);
     cudaStreamCaptureStatus st;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
@@ -199,13 +199,13 @@ int capture_tick_impl(sgc_batch* b) {
 int run_tick_eager(sgc_batch* b) {
     sgc_handle* h = b->h;
     cudaStream_t s = h->stream;
-    enqueue_head(b, s);
+    enqueue_head(b, s, nullptr);
     for (;;) {
-        launch_repair_sweep(h->g, h->sb, SWEEP_INDEP, h->num_sms, s);
-        launch_repair_step(h->g, h->sb, h->num_sms, s, nullptr);
         CK(cudaMemcpyAsync(h->h_rc_out, h->sb.rc, sizeof(RepairCtl), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         if (!h->h_rc_out->cont) break;
+        launch_repair_sweep(h->g, h->sb, SWEEP_INDEP, h->num_sms, s);
+        launch_repair_step(h->g, h->sb, h->num_sms, s, nullptr);
     }
     enqueue_tail(b, s);
     return check_cuda("batch tick");
@@ -367,12 +367,6 @@ int sgc_batch_create(const sgc_batch_graph* graphs, uint32_t count, const sgc_ba
     rethreshold_kernel<<<h->num_sms * 8, 256, 0, h->stream>>>(h->g, const_cast<uint32_t*>(h->g.hdmap), b->d_hdidx,
                                                                b->d_thr);
     CK(cudaMemsetAsync(b->d_dyn, 0, 16, h->stream));
-    // repair control: host fields stay fixed for the batch
-    RepairCtl* hin = h->h_rc_in;
-    hin->mode = SWEEP_INDEP;
-    hin->max_sweeps = 64;
-    hin->force_all = 0;
-    CK(cudaMemcpyAsync(h->sb.rc, hin, 12, cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamCreateWithFlags(&b->qstream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&b->ev0));
     CK(cudaEventCreate(&b->ev1));

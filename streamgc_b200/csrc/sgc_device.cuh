@@ -38,6 +38,7 @@ enum : uint32_t {
     ERR_CHAIN = 1u << 3,          // same-edge ordering words inconsistent with the batch (chain past
                                   // the batch, or an update whose prep record does not match it)
     ERR_RETRY = 1u << 4,          // a color compare-and-swap kept failing past its retry bound
+    ERR_BARRIER = 1u << 6,        // a barrier across a cooperative grid gave up
     ERR_ROW = 1u << 5,            // a row's high-water mark lay past its capacity (scans clamped)
 };
 

@@ -111,10 +111,6 @@ struct sgc_handle {
     uint64_t ring_head = 0;              // consumer: positions gathered (launched)
     uint64_t ring_inflight = 0;          // consumer: end of the last launched gather
     cudaEvent_t ring_done = nullptr;     // recorded after the last gather
-    // SGC_OPT_GRAPH_PUBLISH: the publish captured once per snapshot half
-    cudaGraph_t pub_graph[2] = {nullptr, nullptr};
-    cudaGraphExec_t pub_exec[2] = {nullptr, nullptr};
-    bool pub_graph_failed = false;  // capture failed: the eager publish
     uint64_t launches = 0;          // kernels this handle launched
     uint64_t h2d_bytes = 0, d2h_bytes = 0;  // bytes the library moved across PCIe / C2C
 };
@@ -150,11 +146,10 @@ int sync(sgc_handle* h);
 int compact_dirty(sgc_handle* h, bool force);
 int drain(sgc_handle* h, bool ordered, unsigned long long* failed_counter);
 int set_clean(sgc_handle* h, uint32_t v);
-int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full);
+int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool timed);
 int finish_repair(sgc_handle* h, sgc_repair_report* rep);
 int apply_device(sgc_handle* h, const EdgeUpdate* src, uint32_t n, int mode);
 int ensure_ingest(sgc_handle* h);
-void drop_publish_graphs(sgc_handle* h);
 // Extra layout of a handle that holds several graphs (the batched engine).
 struct CreateExtra {
     const uint32_t* thr_word;  // per 32-vertex word: histogram threshold (null: cfg->histogram_threshold)

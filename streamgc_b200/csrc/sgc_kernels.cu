@@ -57,6 +57,21 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t& total) 
     return x - v;
 }
 
+// One warp's words of a bitmask as list entries, appended at *count.
+__device__ __forceinline__ void list_bits(uint32_t w, uint32_t bits, uint32_t* list, uint32_t* count) {
+    uint32_t total = 0;
+    const uint32_t off = warp_excl_scan(__popc(bits), total);
+    uint32_t base = 0;
+    if (lane_id() == 0 && total) base = atomicAdd(count, total);
+    base = __shfl_sync(FULL, base, 0);
+    uint32_t k = base + off;
+    while (bits) {
+        const int i = __ffs(bits) - 1;
+        bits &= bits - 1;
+        list[k++] = w * 32 + i;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // update kernels
 // ---------------------------------------------------------------------------
@@ -473,17 +488,7 @@ __global__ void dirty_list_kernel(Dev g, uint32_t* list, uint32_t* count) {
         bits = g.dirty[w];
         if (bits) g.dirty[w] = 0;
     }
-    uint32_t total = 0;
-    const uint32_t off = warp_excl_scan(__popc(bits), total);
-    uint32_t base = 0;
-    if (lane_id() == 0 && total) base = atomicAdd(count, total);
-    base = __shfl_sync(FULL, base, 0);
-    uint32_t k = base + off;
-    while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1;
-        list[k++] = w * 32 + b;
-    }
+    list_bits(w, bits, list, count);
 }
 
 void launch_dirty_list(const Dev& g, uint32_t* list, uint32_t* count, cudaStream_t s) {
@@ -768,21 +773,34 @@ void launch_query(const uint16_t* snap, uint32_t n, const uint32_t* v, uint16_t*
 // ---------------------------------------------------------------------------
 //
 // A repair is a loop of sweeps whose state lives in the RepairCtl block on the
-// device: repair_begin_kernel starts it, each sweep reads its index and its
-// vertex set (every vertex, or the worklist b.wl) from there, and
-// repair_step_kernel decides whether another sweep runs. The host either reads
-// the block after each sweep (sgc_repair / sgc_publish) or lets a CUDA-graph
-// while-node run the loop (the batched engine): the kernels are the same.
+// device: repair_begin starts it, each sweep reads its index and its vertex set
+// (every vertex, or the worklist b.wl) from there, and repair_step decides
+// whether another sweep runs. One kernel runs the loop (repair_fused_kernel);
+// sweeps over many vertices, and timed ones, run pass by pass as kernels of their
+// own, between which the host or a CUDA-graph while-node reads the decision.
 
 // list_mode of the per-vertex passes: 0 every vertex, 1 b.wl, 2 as RepairCtl says.
 __device__ __forceinline__ bool use_list(const SweepBufs& b, int list_mode) {
     return list_mode == 2 ? ld_cg(&b.rc->list) != 0 : list_mode == 1;
 }
 
-__global__ void build_items_kernel(Dev g, SweepBufs b, int list_mode) {
+// Warp-collective: vertex x's k work items (k = 0: none).
+__device__ __forceinline__ void append_items(const Dev& g, const SweepBufs& b, uint32_t x, uint32_t k) {
+    uint32_t total = 0;
+    const uint32_t off = warp_excl_scan(k, total);
+    uint32_t wbase = 0;
+    if (lane_id() == 0 && total) wbase = atomicAdd(b.item_count, total);
+    wbase = __shfl_sync(FULL, wbase, 0);
+    if (wbase + off + k > b.item_cap) {
+        if (k) atomicOr(g.err, ERR_LIST_OVERFLOW);
+        return;
+    }
+    for (uint32_t j = 0; j < k; j++) b.items[wbase + off + j] = (unsigned long long)x | ((unsigned long long)j << 32);
+}
+
+__device__ __forceinline__ void build_items(const Dev& g, const SweepBufs& b, int list_mode) {
     const bool list = use_list(b, list_mode);
     const uint32_t lim = list ? *b.wl_count : g.n;
-    const uint32_t tile = b.tile;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < lim; base += stride) {  // warp-uniform trip count
         const uint32_t t = base + threadIdx.x;
@@ -790,20 +808,12 @@ __global__ void build_items_kernel(Dev g, SweepBufs b, int list_mode) {
         if (t < lim) {
             x = list ? b.wl[t] : t;
             const uint32_t len = row_len(g, x);
-            if (len > SWEEP_TINY) k = (len + tile - 1) / tile;
+            if (len > SWEEP_TINY) k = (len + b.tile - 1) / b.tile;
         }
-        uint32_t total = 0;
-        const uint32_t off = warp_excl_scan(k, total);
-        uint32_t wbase = 0;
-        if (lane_id() == 0 && total) wbase = atomicAdd(b.item_count, total);
-        wbase = __shfl_sync(FULL, wbase, 0);
-        if (wbase + off + k > b.item_cap) {
-            if (k) atomicOr(g.err, ERR_LIST_OVERFLOW);
-            continue;
-        }
-        for (uint32_t j = 0; j < k; j++) b.items[wbase + off + j] = (unsigned long long)x | ((unsigned long long)j << 32);
+        append_items(g, b, x, k);
     }
 }
+__global__ void build_items_kernel(Dev g, SweepBufs b, int list_mode) { build_items(g, b, list_mode); }
 void launch_build_items(const Dev& g, const SweepBufs& b, int list_mode, int num_sms, cudaStream_t s) {
     cudaMemsetAsync(b.item_count, 0, sizeof(uint32_t), s);
     uint32_t blocks = (g.n + 255) / 256;
@@ -833,15 +843,16 @@ __device__ __forceinline__ void item_bounds(const Dev& g, const SweepBufs& b, un
     e = s + b.tile < re ? s + b.tile : re;
 }
 
-// Warp per item: up to b.tile live slots of one row. Nothing in the graph
-// changes during a sweep, so loads take the read-only path. Each lane keeps two
+// Warp per item: up to b.tile live slots of one row. State words and conflict
+// flags are read with plain loads throughout the sweep's passes: in the
+// one-kernel repair they change between passes. Each lane keeps two
 // 16-byte slot loads and their eight state gathers in flight per round.
 // SYM: accumulate the mirror checksum of rows whose graph wants it. PUSH
 // (independent-set rule): a same-colored neighbor that loses to x (lower
 // priority) is marked for the next sweep, which decides it from its own row.
 template <bool SYM, bool PUSH>
-__device__ __forceinline__ void sweep_items_body(const Dev& g, const SweepBufs& b) {
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+__device__ __forceinline__ void sweep_items_body(const Dev& g, const SweepBufs& b, uint32_t nb) {
+    const uint32_t warps = (nb * blockDim.x) >> 5;
     const uint32_t lane = lane_id();
     const uint32_t cnt = *b.item_count;
     for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < cnt; k += warps) {
@@ -850,7 +861,7 @@ __device__ __forceinline__ void sweep_items_body(const Dev& g, const SweepBufs& 
         item_bounds(g, b, b.items[k], x, s, e);
         GraphCtl* gc = SYM ? &g.gctl[graph_of(g, x)] : nullptr;
         const bool symx = SYM && gc->full && ld_cg(&gc->asym);
-        const uint32_t myc = color_of(__ldg(g.st + x));
+        const uint32_t myc = color_of(g.st[x]);
         const uint32_t mydeg = (g.abl & ABL_LIVE_DEG) ? row_len(g, x) : __ldg(g.deg + x);
         uint32_t lo = 0, hi = 0;
         unsigned long long sym = 0;
@@ -867,7 +878,7 @@ __device__ __forceinline__ void sweep_items_body(const Dev& g, const SweepBufs& 
                 const uint64_t p = (t < 4 ? i0 : i1) + (t & 3);
                 const bool in = p >= s && p < e && v[t] < g.n;
                 v[t] = in ? v[t] : INV;
-                nc[t] = in ? color_of(__ldg(g.st + v[t])) : 0u;
+                nc[t] = in ? color_of(g.st[v[t]]) : 0u;
             }
 #pragma unroll
             for (int t = 0; t < 8; t++) {
@@ -903,16 +914,20 @@ __device__ __forceinline__ bool want_sym(const SweepBufs& b, int sym_mode) {
     return sym_mode == 2 && ld_cg(&b.rc->it) == 0 && ld_cg(&b.rc->any_sym) != 0;
 }
 
-__global__ void __launch_bounds__(256, 5) sweep_items_kernel(Dev g, SweepBufs b, int mode, int sym_mode) {
+__device__ __forceinline__ void sweep_items(const Dev& g, const SweepBufs& b, int mode, int sym_mode, uint32_t nb) {
     const bool sym = want_sym(b, sym_mode);
     const bool push = mode == SWEEP_INDEP;
     if (push) {
-        if (sym) sweep_items_body<true, true>(g, b);
-        else sweep_items_body<false, true>(g, b);
+        if (sym) sweep_items_body<true, true>(g, b, nb);
+        else sweep_items_body<false, true>(g, b, nb);
     } else {
-        if (sym) sweep_items_body<true, false>(g, b);
-        else sweep_items_body<false, false>(g, b);
+        if (sym) sweep_items_body<true, false>(g, b, nb);
+        else sweep_items_body<false, false>(g, b, nb);
     }
+}
+
+__global__ void __launch_bounds__(256, 5) sweep_items_kernel(Dev g, SweepBufs b, int mode, int sym_mode) {
+    sweep_items(g, b, mode, sym_mode, gridDim.x);
 }
 
 // One vertex of the finalize pass (warp-collective: every lane calls it; `valid`
@@ -945,10 +960,10 @@ __device__ __forceinline__ void piece_ids(const Dev& g, uint64_t s, uint64_t e, 
 }
 
 __device__ __forceinline__ void finalize_one(const Dev& g, const SweepBufs& b, int mode, bool valid, uint32_t x,
-                                             bool with_sym, bool push) {
+                                             bool with_sym, bool push, unsigned long long& live_sum) {
     bool fac_needed = false, pend = false, need = false;
     uint32_t pend_word = 0;
-    unsigned long long sym = 0, live = 0;
+    unsigned long long sym = 0;
     if (valid) {
         if (with_sym) {
             const GraphCtl& gc = g.gctl[graph_of(g, x)];
@@ -956,11 +971,11 @@ __device__ __forceinline__ void finalize_one(const Dev& g, const SweepBufs& b, i
         }
         const uint32_t len = row_len(g, x);
         const uint32_t hd = __ldg(g.hdmap + x);
-        const uint32_t w = __ldg(g.st + x);
+        const uint32_t w = g.st[x];
         const uint16_t myc = color_of(w);
         unsigned long long bits = 0;
         bool conf = false;
-        live = len;
+        live_sum += len;
         if (len <= SWEEP_TINY) {
             const uint32_t mydeg = (g.abl & ABL_LIVE_DEG) ? len : __ldg(g.deg + x);
             uint32_t lo = 0, hi = 0;
@@ -969,7 +984,7 @@ __device__ __forceinline__ void finalize_one(const Dev& g, const SweepBufs& b, i
                 uint32_t y[kPieceIds], sw[kPieceIds];
                 piece_ids<true>(g, s, s + kPiece < e0 ? s + kPiece : e0, y);
 #pragma unroll
-                for (int t = 0; t < kPieceIds; t++) sw[t] = y[t] != INV ? __ldg(g.st + y[t]) : 0u;
+                for (int t = 0; t < kPieceIds; t++) sw[t] = y[t] != INV ? g.st[y[t]] : 0u;
 #pragma unroll
                 for (int t = 0; t < kPieceIds; t++) {
                     const uint32_t ng = y[t];
@@ -1023,16 +1038,7 @@ __device__ __forceinline__ void finalize_one(const Dev& g, const SweepBufs& b, i
             }
         }
     }
-    for (int off = 16; off > 0; off >>= 1) live += __shfl_xor_sync(FULL, live, off);
     if (sym) atomicAdd(&g.gctl[graph_of(g, x)].sym, sym);  // per lane: the lanes' rows may sit in different graphs
-    const unsigned long long nv = __popc(__ballot_sync(FULL, valid));
-    if (lane_id() == 0) {
-        if (live) {
-            atomicAdd(b.live, live);
-            atomicAdd(b.swept, live);
-        }
-        if (nv) atomicAdd(b.swept + 1, nv);
-    }
     if (mode == SWEEP_INDEP) {
         const uint32_t ni = warp_append(b.need_count, need);
         if (need) b.need_v[ni] = x;
@@ -1048,27 +1054,49 @@ __device__ __forceinline__ void finalize_one(const Dev& g, const SweepBufs& b, i
     }
 }
 
+// The live entries and vertices a pass visited, summed per warp over the whole
+// pass: one atomic per warp and counter.
+__device__ __forceinline__ void count_visits(const SweepBufs& b, unsigned long long live, uint32_t seen) {
+    for (int off = 16; off > 0; off >>= 1) live += __shfl_xor_sync(FULL, live, off);
+    seen = __reduce_add_sync(FULL, seen);
+    if (lane_id() != 0 || !seen) return;
+    if (live) {
+        atomicAdd(b.live, live);
+        atomicAdd(b.swept, live);
+    }
+    atomicAdd(b.swept + 1, (unsigned long long)seen);
+}
+
 // Thread per vertex (every vertex, or the worklist).
-__global__ void __launch_bounds__(256, 3) sweep_finalize_kernel(Dev g, SweepBufs b, int mode, int list_mode,
-                                                             int sym_mode) {
+__device__ __forceinline__ void sweep_finalize(const Dev& g, const SweepBufs& b, int mode, int list_mode, int sym_mode, uint32_t nb) {
     const bool list = use_list(b, list_mode);
     const uint32_t lim = list ? *b.wl_count : g.n;
-    const uint32_t stride = gridDim.x * blockDim.x;
+    const uint32_t stride = nb * blockDim.x;
     const bool sym = want_sym(b, sym_mode);
     const bool push = mode == SWEEP_INDEP;
+    unsigned long long live = 0;
+    uint32_t seen = 0;
     for (uint32_t base = blockIdx.x * blockDim.x; base < lim; base += stride) {  // warp-uniform trip count
         const uint32_t t = base + threadIdx.x;
         const bool valid = t < lim;
-        finalize_one(g, b, mode, valid, valid ? (list ? b.wl[t] : t) : 0, sym, push);
+        seen += valid;
+        finalize_one(g, b, mode, valid, valid ? (list ? b.wl[t] : t) : 0, sym, push, live);
     }
+    count_visits(b, live, seen);
+}
+__global__ void __launch_bounds__(256, 3) sweep_finalize_kernel(Dev g, SweepBufs b, int mode, int list_mode,
+                                                             int sym_mode) {
+    sweep_finalize(g, b, mode, list_mode, sym_mode, gridDim.x);
 }
 
 // Warp per vertex whose new color needs the histogram row or the >64 scan;
 // colors read are the start-of-sweep ones (nothing is committed yet).
-__global__ void __launch_bounds__(256) sweep_fac_kernel(Dev g, SweepBufs b) {
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+// (The scratch of the exact selection serves eight warps of a block.)
+__device__ __forceinline__ void sweep_fac(const Dev& g, const SweepBufs& b, uint32_t nb) {
+    if (threadIdx.x >= 256) return;
+    const uint32_t warps = nb * 8;
     const uint32_t cnt = *b.fac_count;
-    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < cnt; k += warps) {
+    for (uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5); k < cnt; k += warps) {
         const uint32_t x = b.fac_v[k];
         const uint32_t w = ld_cg(g.st + x);
         const uint16_t c = warp_fac(g, x, g.st);
@@ -1080,16 +1108,18 @@ __global__ void __launch_bounds__(256) sweep_fac_kernel(Dev g, SweepBufs b) {
         __syncwarp();
     }
 }
+__global__ void __launch_bounds__(256) sweep_fac_kernel(Dev g, SweepBufs b) { sweep_fac(g, b, gridDim.x); }
 
 // Independent-set selection, step 1: warp per item (chunk) of a conflicted
 // row. Sets the row's blocked flag (acc_fl) when a conflicted neighbor in the
 // chunk ranks above it; for a histogram-class row whose neighbors take every
 // color 1..64 (acc_bm, from the sweep) it also gathers the taken colors 65..2047
 // into the row's words of b.hiused. Colors are the start-of-sweep ones.
-__global__ void __launch_bounds__(256, 5) indep_items_kernel(Dev g, SweepBufs b) {
-    __shared__ uint32_t s_used[8][64];
+template <int WARPS>
+__device__ __forceinline__ void indep_items(const Dev& g, const SweepBufs& b, uint32_t nb) {
+    __shared__ uint32_t s_used[WARPS][64];
     uint32_t* used = s_used[threadIdx.x >> 5];
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t warps = (nb * blockDim.x) >> 5;
     const uint32_t lane = lane_id();
     const uint32_t cnt = *b.item_count;
     const uint32_t salt = sweep_salt(ld_cg(&b.rc->it));
@@ -1098,13 +1128,14 @@ __global__ void __launch_bounds__(256, 5) indep_items_kernel(Dev g, SweepBufs b)
     __syncwarp();
     for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < cnt; k += warps) {
         const unsigned long long it = b.items[k];
-        if (!__ldg(b.needf + (uint32_t)it)) continue;
-        if (ld_cg(b.acc_fl + (uint32_t)it)) continue;  // another chunk already found it blocked
         uint32_t x;
         uint64_t s, e;
         item_bounds(g, b, it, x, s, e);
-        const uint32_t hd = __ldg(g.hdmap + x);
-        const bool full = hd != EMPTY && g.exact && ~b.acc_bm[x] == 0ull;
+        // the row's words in one round trip, before the first is tested
+        const uint32_t hd = __ldg(g.hdmap + x), met = ld_cg(b.acc_fl + x);
+        const unsigned long long mask = b.acc_bm[x];
+        const bool full = hd != EMPTY && g.exact && ~mask == 0ull;
+        if (!b.needf[x] || met) continue;  // not conflicted, or another chunk already found it blocked
         const uint32_t base = g.gctl[graph_of(g, x)].base;  // ranks use the graph's own ids
         const unsigned long long rx = sel_rank(x - base, salt);
         bool blocked = false;
@@ -1121,8 +1152,8 @@ __global__ void __launch_bounds__(256, 5) indep_items_kernel(Dev g, SweepBufs b)
                 const uint64_t p = (t < 4 ? i0 : i1) + (t & 3);
                 const bool in = p >= s && p < e && v[t] < g.n && v[t] != x;
                 v[t] = in ? v[t] : INV;
-                nf[t] = in ? __ldg(b.needf + v[t]) : (uint8_t)0;
-                nc[t] = (in && full) ? color_of(__ldg(g.st + v[t])) : 0u;
+                nf[t] = in ? b.needf[v[t]] : (uint8_t)0;
+                nc[t] = (in && full) ? color_of(g.st[v[t]]) : 0u;
             }
 #pragma unroll
             for (int t = 0; t < 8; t++) {
@@ -1146,6 +1177,8 @@ __global__ void __launch_bounds__(256, 5) indep_items_kernel(Dev g, SweepBufs b)
     }
 }
 
+__global__ void __launch_bounds__(256, 5) indep_items_kernel(Dev g, SweepBufs b) { indep_items<8>(g, b, gridDim.x); }
+
 // Independent-set selection, step 2: thread per conflicted vertex. A row of at
 // most SWEEP_TINY slots checks its neighbors here; longer rows read step 1's
 // flag. An unblocked vertex takes the first color its neighbors leave free:
@@ -1153,10 +1186,10 @@ __global__ void __launch_bounds__(256, 5) indep_items_kernel(Dev g, SweepBufs b)
 // (histogram-class rows), else through the warp scan of sweep_fac_kernel
 // (bitmap rows whose 64 low colors are all taken). Blocked vertices are marked
 // for the next sweep.
-__global__ void __launch_bounds__(256) indep_decide_kernel(Dev g, SweepBufs b) {
+__device__ __forceinline__ void indep_decide(const Dev& g, const SweepBufs& b, uint32_t nb) {
     const uint32_t cnt = *b.need_count;
     const uint32_t salt = sweep_salt(ld_cg(&b.rc->it));
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += nb * blockDim.x) {
         const uint32_t x = b.need_v[t];
         const uint32_t len = row_len(g, x);
         bool blocked = false;
@@ -1169,7 +1202,7 @@ __global__ void __launch_bounds__(256) indep_decide_kernel(Dev g, SweepBufs b) {
                 uint8_t nf[kPieceIds];
                 piece_ids<true>(g, s, s + kPiece < e0 ? s + kPiece : e0, y);
 #pragma unroll
-                for (int t = 0; t < kPieceIds; t++) nf[t] = (y[t] != INV && y[t] != x) ? __ldg(b.needf + y[t]) : 0;
+                for (int t = 0; t < kPieceIds; t++) nf[t] = (y[t] != INV && y[t] != x) ? b.needf[y[t]] : 0;
 #pragma unroll
                 for (int t = 0; t < kPieceIds; t++)
                     if (nf[t] && sel_rank(y[t] - base, salt) > rx) blocked = true;
@@ -1208,16 +1241,18 @@ __global__ void __launch_bounds__(256) indep_decide_kernel(Dev g, SweepBufs b) {
     }
 }
 
+__global__ void __launch_bounds__(256) indep_decide_kernel(Dev g, SweepBufs b) { indep_decide(g, b, gridDim.x); }
+
 // Writes the chosen colors and clears the recolored vertices' conflict flags.
 // Reference rule (TIER1): marks each recolored vertex and, for rows of at most
 // SWEEP_TINY slots, its neighbors for the next worklist (longer rows: per item
 // in mark_items_kernel). Independent-set rule: ORs the new color into the
 // neighbors' bitmaps instead (the next sweep needs no neighbor of a recolored
 // vertex: under that rule a recolor creates no conflict).
-__global__ void sweep_commit_kernel(Dev g, SweepBufs b, int mode) {
+__device__ __forceinline__ void sweep_commit(const Dev& g, const SweepBufs& b, int mode, uint32_t nb) {
     const uint32_t cnt = *b.pend_count;
     const bool incr = mode == SWEEP_INDEP;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += nb * blockDim.x) {
         const uint32_t x = b.pend_v[k];
         const uint32_t nw = b.pend_w[k];
         g.st[x] = nw;
@@ -1243,11 +1278,13 @@ __global__ void sweep_commit_kernel(Dev g, SweepBufs b, int mode) {
     }
 }
 
+__global__ void sweep_commit_kernel(Dev g, SweepBufs b, int mode) { sweep_commit(g, b, mode, gridDim.x); }
+
 // Warp per item of the last sweep whose row was recolored: marks the
 // neighbors in the item's slots (reference rule) or ORs the row's new color
 // into their bitmaps (independent-set rule).
-__global__ void __launch_bounds__(256) mark_items_kernel(Dev g, SweepBufs b) {
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+__device__ __forceinline__ void mark_items(const Dev& g, const SweepBufs& b, uint32_t nb) {
+    const uint32_t warps = (nb * blockDim.x) >> 5;
     const uint32_t lane = lane_id();
     const uint32_t cnt = *b.item_count;
     const bool incr = ld_cg(&b.rc->mode) == SWEEP_INDEP;
@@ -1270,38 +1307,40 @@ __global__ void __launch_bounds__(256) mark_items_kernel(Dev g, SweepBufs b) {
     }
 }
 
-// Turns a bitmask into a list (appending at *count) and clears it; `clear2`
-// (optional) is cleared alongside. With `keep` zero the bits are only cleared.
-__global__ void collect_bits_kernel(uint32_t n, uint32_t* bits_arr, uint32_t* clear2, uint32_t* list, uint32_t* count,
-                                    const uint32_t* keep) {
+__global__ void __launch_bounds__(256) mark_items_kernel(Dev g, SweepBufs b) { mark_items(g, b, gridDim.x); }
+
+// The next worklist: the marked vertices; clears the marks.
+__device__ __forceinline__ void collect_marks(const Dev& g, const SweepBufs& b, uint32_t nb) {
+    const uint32_t nw = (g.n + 31) / 32;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < nw; base += nb * blockDim.x) {
+        const uint32_t w = base + threadIdx.x;
+        uint32_t bits = 0;
+        if (w < nw) {
+            bits = b.wmark[w];
+            if (bits) b.wmark[w] = 0;
+        }
+        list_bits(w, bits, b.wl, b.wl_count);
+        uint32_t k = 0;  // the work items they will make
+        for (uint32_t r = bits; r; r &= r - 1) {
+            const uint32_t len = row_len(g, w * 32 + (__ffs(r) - 1));
+            if (len > SWEEP_TINY) k += (len + b.tile - 1) / b.tile;
+        }
+        k = __reduce_add_sync(FULL, k);
+        if (k && lane_id() == 0) atomicAdd(b.next_items, k);
+    }
+}
+// (and the recolored bits, which nothing reads any more)
+__global__ void collect_marks_kernel(Dev g, SweepBufs b) {
     const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t nw = (n + 31) / 32;
-    const bool k_on = keep == nullptr || ld_cg(keep) != 0;
-    uint32_t bits = 0;
-    if (w < nw) {
-        bits = bits_arr[w];
-        if (bits) bits_arr[w] = 0;
-        if (clear2 && clear2[w]) clear2[w] = 0;
-    }
-    if (!k_on) bits = 0;
-    uint32_t total = 0;
-    const uint32_t off = warp_excl_scan(__popc(bits), total);
-    uint32_t base = 0;
-    if (lane_id() == 0 && total) base = atomicAdd(count, total);
-    base = __shfl_sync(FULL, base, 0);
-    uint32_t k = base + off;
-    while (bits) {
-        const int i = __ffs(bits) - 1;
-        bits &= bits - 1;
-        list[k++] = w * 32 + i;
-    }
+    if (w < (g.n + 31) / 32 && b.rbits[w]) b.rbits[w] = 0;
+    collect_marks(g, b, gridDim.x);
 }
 
 void launch_next_worklist(const Dev& g, const SweepBufs& b, int num_sms, cudaStream_t s) {
     mark_items_kernel<<<num_sms * 8, 256, 0, s>>>(g, b);
     cudaMemsetAsync(b.wl_count, 0, sizeof(uint32_t), s);
     const uint32_t nw = (g.n + 31) / 32;
-    collect_bits_kernel<<<(nw + 255) / 256, 256, 0, s>>>(g.n, b.wmark, b.rbits, b.wl, b.wl_count, nullptr);
+    collect_marks_kernel<<<(nw + 255) / 256, 256, 0, s>>>(g, b);
 }
 
 void launch_sweep(const Dev& g, const SweepBufs& b, SweepMode mode, int list_mode, int sym_mode, int num_sms,
@@ -1333,7 +1372,7 @@ void launch_sweep(const Dev& g, const SweepBufs& b, SweepMode mode, int list_mod
 // not end proper, its rows may miss mirror entries, or the host forces it),
 // else the vertices its updates touched since the last repair: every new
 // conflict then has a touched endpoint. One block.
-__global__ void repair_begin_kernel(Dev g, SweepBufs b) {
+__device__ __forceinline__ void repair_begin(const Dev& g, const SweepBufs& b) {
     RepairCtl& rc = *b.rc;
     const bool indep = rc.mode == SWEEP_INDEP;
     uint32_t any_sym = 0, any_incr = 0;
@@ -1368,35 +1407,30 @@ __global__ void repair_begin_kernel(Dev g, SweepBufs b) {
     }
 }
 
+__global__ void repair_begin_kernel(Dev g, SweepBufs b) { repair_begin(g, b); }
+
 // First worklist of an independent-set repair: every vertex of the graphs
 // repaired in full, the touched vertices of the others; clears the touched
 // marks. Thread per 32-vertex word.
-__global__ void seed_worklist_kernel(Dev g, SweepBufs b) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void seed_worklist(const Dev& g, const SweepBufs& b, uint32_t nb) {
     const uint32_t nw = (g.n + 31) / 32;
-    uint32_t bits = 0;
-    if (w < nw) {
-        const uint32_t t = g.touched[w];
-        if (t) g.touched[w] = 0;
-        if (g.gctl[g.gidw ? g.gidw[w] : 0u].full) {
-            const uint32_t left = g.n - w * 32;
-            bits = left >= 32 ? FULL : (1u << left) - 1u;
-        } else {
-            bits = t;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < nw; base += nb * blockDim.x) {
+        const uint32_t w = base + threadIdx.x;
+        uint32_t bits = 0;
+        if (w < nw) {
+            const uint32_t t = g.touched[w];
+            if (t) g.touched[w] = 0;
+            if (g.gctl[g.gidw ? g.gidw[w] : 0u].full) {
+                const uint32_t left = g.n - w * 32;
+                bits = left >= 32 ? FULL : (1u << left) - 1u;
+            } else {
+                bits = t;
+            }
         }
-    }
-    uint32_t total = 0;
-    const uint32_t off = warp_excl_scan(__popc(bits), total);
-    uint32_t base = 0;
-    if (lane_id() == 0 && total) base = atomicAdd(b.wl_count, total);
-    base = __shfl_sync(FULL, base, 0);
-    uint32_t k = base + off;
-    while (bits) {
-        const int i = __ffs(bits) - 1;
-        bits &= bits - 1;
-        b.wl[k++] = w * 32 + i;
+        list_bits(w, bits, b.wl, b.wl_count);
     }
 }
+__global__ void seed_worklist_kernel(Dev g, SweepBufs b) { seed_worklist(g, b, gridDim.x); }
 
 // After each sweep: reads the counts, decides whether another sweep runs,
 // advances the index. Reference rule (TIER1): stop at 0 conflicts, after 3
@@ -1406,7 +1440,7 @@ __global__ void seed_worklist_kernel(Dev g, SweepBufs b) {
 // sweep a graph whose checksum came out 0 is known mirror-complete; when the
 // loop ends every graph records whether it ended proper. `cond` (graph mode):
 // the while-node's handle receives the decision. One block.
-__global__ void repair_step_kernel(Dev g, SweepBufs b, cudaGraphConditionalHandle cond, int has_cond) {
+__device__ __forceinline__ void repair_step(const Dev& g, const SweepBufs& b) {
     RepairCtl& rc = *b.rc;
     __shared__ uint32_t s_stop;
     const bool indep = rc.mode == SWEEP_INDEP;
@@ -1445,10 +1479,11 @@ __global__ void repair_step_kernel(Dev g, SweepBufs b, cudaGraphConditionalHandl
         }
         rc.done = done ? 1u : 0u;
         rc.list = (indep || rc.sym == 0) ? 1u : 0u;
+        rc.swept[0] = b.swept[0];
+        rc.swept[1] = b.swept[1];
         rc.it += 1;
         rc.cont = (!stop && rc.it < rc.max_sweeps) ? 1u : 0u;
         s_stop = rc.cont ? 0u : 1u;
-        if (has_cond) cudaGraphSetConditional(cond, rc.cont);
     }
     __syncthreads();
     if (s_stop) {
@@ -1466,6 +1501,11 @@ __global__ void repair_step_kernel(Dev g, SweepBufs b, cudaGraphConditionalHandl
     }
 }
 
+__global__ void repair_step_kernel(Dev g, SweepBufs b, cudaGraphConditionalHandle cond, int has_cond) {
+    repair_step(g, b);
+    if (has_cond && threadIdx.x == 0) cudaGraphSetConditional(cond, b.rc->cont);
+}
+
 void launch_repair_begin(const Dev& g, const SweepBufs& b, SweepMode mode, int num_sms, cudaStream_t s) {
     repair_begin_kernel<<<1, 256, 0, s>>>(g, b);
     if (mode == SWEEP_INDEP && g.touched) {
@@ -1473,6 +1513,262 @@ void launch_repair_begin(const Dev& g, const SweepBufs& b, SweepMode mode, int n
         seed_worklist_kernel<<<(nw + 255) / 256, 256, 0, s>>>(g, b);
     }
     (void)num_sms;
+}
+
+// ---------------------------------------------------------------------------
+// the repair as one kernel
+// ---------------------------------------------------------------------------
+//
+// Most repairs are short: an epoch's worklist of some ten thousand vertices, two
+// to ten sweeps of a few microseconds of work each. As fourteen launches per
+// sweep, and a host or while-node round trip, a sweep took 55 us (epochs of 4,096
+// updates on a mesh of 24,001 vertices: 245 us, now 152). One cooperative launch
+// with a block per SM runs the same passes with a barrier across the grid (2 us)
+// between them and leaves out the passes that have nothing to do; a short
+// worklist is left to kTailBlocks blocks, whose barrier costs less.
+//   kTailList, kTailItems: what sixteen blocks finish in one or two rounds of
+// their warps. Sweeps of a power-law graph of 2 M vertices there: 40 us against
+// 49 on the whole grid.
+//   kFusedMax: the passes share one register budget (80: 24 warps per SM), so a
+// sweep over many vertices, where the item passes' 40 warps per SM pay and a
+// launch costs little, is left to the kernels above.
+constexpr uint32_t kFusedThreads = 768;
+constexpr uint32_t kTailBlocks = 16, kTailList = 2048, kTailItems = 768;
+
+// The first `nb` blocks of the grid meet. A thread's writes before the barrier
+// are seen after it by plain loads in all of them. Round by round the arrivals
+// only grow by nb, so a round is over when they reach the next multiple. The
+// wait is bounded (seconds): false means a block is missing, and the caller
+// returns.
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+struct GridSync {
+    GridBar* bar;
+    uint32_t* err;
+    uint32_t nb;
+    unsigned long long due = 0, serials = 0;  // thread 0: arrivals and serial sections awaited so far
+
+    __device__ __forceinline__ GridSync(GridBar* p, uint32_t* e) : bar(p), err(e), nb(gridDim.x) {}
+    __device__ __forceinline__ bool wait(const unsigned long long* word, unsigned long long target) {
+        for (uint32_t polls = 0; ld_acquire(word) < target; polls++) {
+            if (polls > 2000u) __nanosleep(200);
+            if (polls >= (1u << 25) || *(volatile uint32_t*)&bar->failed) {
+                *(volatile uint32_t*)&bar->failed = 1;
+                atomicOr(err, ERR_BARRIER);
+                return false;
+            }
+        }
+        return true;
+    }
+    __device__ __forceinline__ void arrive() {
+        fence_gpu();
+        atomicAdd(&bar->count, 1ull);
+        due += nb;
+    }
+    __device__ __forceinline__ bool operator()() {
+        bool ok = true;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            arrive();
+            ok = wait(&bar->count, due);
+        }
+        return __syncthreads_and(ok);
+    }
+    // The same, where block 0 runs `last` when all have arrived, before any goes on.
+    template <class F>
+    __device__ __forceinline__ bool serial(F last) {
+        bool ok = true;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            arrive();
+            ok = blockIdx.x == 0 ? wait(&bar->count, due) : wait(&bar->gen, ++serials);
+        }
+        if (!__syncthreads_and(ok)) return false;
+        if (blockIdx.x == 0) {
+            last();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                fence_gpu();
+                atomicAdd(&bar->gen, 1ull);
+            }
+        }
+        return true;
+    }
+    // The last block to leave makes the words zero for the next launch.
+    __device__ __forceinline__ void leave() {
+        __syncthreads();
+        if (threadIdx.x == 0 && atomicAdd(&bar->left, 1u) == gridDim.x - 1) {
+            bar->count = 0;
+            bar->gen = 0;
+            bar->left = 0;
+        }
+    }
+};
+
+// First pass of a sweep: work items for the long rows, the short rows whole.
+__device__ __forceinline__ void sweep_short(const Dev& g, const SweepBufs& b, int mode, bool list, uint32_t lim,
+                                            bool sym, uint32_t nb) {
+    unsigned long long live = 0;
+    uint32_t seen = 0;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < lim; base += nb * blockDim.x) {
+        const uint32_t t = base + threadIdx.x;
+        uint32_t k = 0, x = 0;
+        if (t < lim) {
+            x = list ? b.wl[t] : t;
+            const uint32_t len = row_len(g, x);
+            if (len > SWEEP_TINY) k = (len + b.tile - 1) / b.tile;
+        }
+        append_items(g, b, x, k);
+        const bool valid = t < lim && k == 0;
+        seen += valid;
+        finalize_one(g, b, mode, valid, x, sym, mode == SWEEP_INDEP, live);
+    }
+    count_visits(b, live, seen);
+}
+// After the items: the long rows (each at its first item).
+__device__ __forceinline__ void sweep_long(const Dev& g, const SweepBufs& b, int mode, uint32_t items, bool sym,
+                                           uint32_t nb) {
+    unsigned long long live = 0;
+    uint32_t seen = 0;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < items; base += nb * blockDim.x) {
+        const uint32_t t = base + threadIdx.x;
+        const unsigned long long it = t < items ? b.items[t] : ~0ull;
+        const bool valid = (it >> 32) == 0;
+        seen += valid;
+        finalize_one(g, b, mode, valid, (uint32_t)it, sym, mode == SWEEP_INDEP, live);
+    }
+    count_visits(b, live, seen);
+}
+
+// False: a barrier gave up.
+__device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, GridSync& sync, int start,
+                                             const RepairIn& in, uint32_t most) {
+    RepairCtl& rc = *b.rc;
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t nw = (g.n + 31) / 32;
+    if (start) {  // no marks, no vertex conflicted
+        const uint32_t threads = gridDim.x * blockDim.x;
+        for (uint32_t w = tid; w < nw; w += threads) {
+            b.wmark[w] = 0;
+            b.rbits[w] = 0;
+        }
+        for (uint32_t x = tid; x < g.n; x += threads) b.needf[x] = 0;
+    }
+    auto reset = [&] {
+        if (threadIdx.x == 0) {
+            *b.item_count = 0;
+            *b.pend_count = 0;
+            *b.fac_count = 0;
+            *b.need_count = 0;
+        }
+    };
+    if (!sync.serial([&] {
+            reset();
+            if (threadIdx.x == 0) *b.next_items = NONE32;  // not counted for the first list
+            if (start) {
+                if (threadIdx.x == 0) {
+                    rc.mode = in.mode;
+                    rc.max_sweeps = in.max_sweeps;
+                    rc.force_all = in.force_all;
+                }
+                __syncthreads();
+                repair_begin(g, b);
+            }
+        }))
+        return false;
+    const int mode = (int)rc.mode;
+    const bool indep = mode == SWEEP_INDEP;
+    if (start && indep) {
+        seed_worklist(g, b, sync.nb);
+        if (!sync()) return false;
+    }
+    bool recolored = false;  // bits set in b.rbits
+    for (;;) {
+        if (recolored)
+            for (uint32_t w = tid; w < nw; w += sync.nb * blockDim.x) b.rbits[w] = 0;
+        const bool list = rc.list != 0;
+        const uint32_t lim = list ? *b.wl_count : g.n;
+        if (!rc.cont || lim > most) return true;
+        if (sync.nb > kTailBlocks) {
+            if (lim <= kTailList && *b.next_items <= kTailItems) {
+                sync.nb = kTailBlocks;
+                if (blockIdx.x >= kTailBlocks) return true;
+            }
+        } else if (lim > 4 * kTailList || *b.next_items > 4 * kTailItems) {
+            return true;  // grown again: another launch goes on
+        }
+        const uint32_t nb = sync.nb;
+        const bool sym = want_sym(b, 2);
+        sweep_short(g, b, mode, list, lim, sym, nb);
+        if (!sync()) return false;
+        if (tid == 0) {  // every block has read them
+            *b.wl_count = 0;
+            *b.next_items = 0;
+        }
+        const uint32_t items = *b.item_count < b.item_cap ? *b.item_count : b.item_cap;
+        if (items) {
+            sweep_items(g, b, mode, 2, nb);
+            if (!sync()) return false;
+            sweep_long(g, b, mode, items, sym, nb);
+            if (!sync()) return false;
+        }
+        if (indep && *b.need_count) {
+            if (items) {
+                indep_items<kFusedThreads / 32>(g, b, nb);
+                if (!sync()) return false;
+            }
+            indep_decide(g, b, nb);
+            if (!sync()) return false;
+        }
+        if (*b.fac_count) {
+            sweep_fac(g, b, nb);
+            if (!sync()) return false;
+        }
+        recolored = *b.pend_count != 0;
+        if (recolored) {
+            sweep_commit(g, b, mode, nb);
+            if ((items || !indep) && !sync()) return false;  // else the commit marks nothing and sets no bit that is read
+            if (items) {
+                mark_items(g, b, nb);
+                if (!indep && !sync()) return false;
+            }
+        }
+        collect_marks(g, b, nb);
+        if (!sync.serial([&] {
+                repair_step(g, b);
+                __syncthreads();
+                reset();
+            }))
+            return false;
+    }
+}
+__global__ void __launch_bounds__(kFusedThreads, 1) repair_fused_kernel(Dev g, SweepBufs b, int start, RepairIn in,
+                                                                        uint32_t most,
+                                                                        cudaGraphConditionalHandle cond,
+                                                                        int has_cond) {
+    GridSync sync(b.bar, g.err);
+    const bool ok = repair_fused(g, b, sync, start, in, most);
+    sync.leave();
+    if (has_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, ok ? b.rc->cont : 0u);
+}
+
+void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start, int num_sms, cudaStream_t s,
+                         const cudaGraphConditionalHandle* cond) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(num_sms);
+    cfg.blockDim = dim3(kFusedThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, repair_fused_kernel, g, b, start ? 1 : 0, start ? *start : RepairIn{}, kFusedMax,
+                       cond ? *cond : (cudaGraphConditionalHandle)0, cond ? 1 : 0);
 }
 
 void launch_repair_sweep(const Dev& g, const SweepBufs& b, SweepMode mode, int num_sms, cudaStream_t s,

@@ -32,6 +32,19 @@ struct RepairCtl {
     uint32_t pad[3];
     unsigned long long sym;   // nonzero: some graph's first-sweep checksum was not 0
     unsigned long long live;  // first sweep's live entries
+    unsigned long long swept[2];  // live entries and vertices visited by the sweeps so far
+};
+// The host's fields of a repair that repair_fused_kernel starts.
+struct RepairIn {
+    uint32_t mode, max_sweeps, force_all;
+};
+
+// Barrier across the blocks of a cooperative launch (one per handle).
+struct GridBar {
+    unsigned long long count;  // arrivals of this launch
+    unsigned long long gen;    // serial sections of this launch that ended
+    uint32_t left;             // blocks that left
+    uint32_t failed;
 };
 
 // Per-sweep work state: warp items for rows longer than SWEEP_TINY, per-vertex
@@ -43,6 +56,7 @@ struct SweepBufs {
     uint32_t tile;               // slots per item (repair tile width, >= SWEEP_CH_MIN)
     uint32_t G;                  // graphs of the handle (entries of g.gctl)
     RepairCtl* rc;
+    GridBar* bar;
     unsigned long long* acc_bm;  // OR of neighbor colors 1..64, per vertex
     uint32_t* acc_fl;            // bit0: a same-colored neighbor has higher priority
     uint32_t* pend_v;            // Jacobi commit list
@@ -55,6 +69,7 @@ struct SweepBufs {
     uint32_t* wmark;             // bitmask
     uint32_t* wl;
     uint32_t* wl_count;
+    uint32_t* next_items;        // work items the next worklist will make
     unsigned long long* swept;   // [0] live entries, [1] vertices visited by the sweeps since reset
     // independent-set sweeps: conflicted vertices of the current sweep
     uint8_t* needf;              // per vertex: conflicted (or uncolored with neighbors) at the last visit
@@ -147,6 +162,14 @@ void launch_repair_sweep(const Dev& g, const SweepBufs& b, SweepMode mode, int n
                          cudaEvent_t* phase = nullptr);
 void launch_repair_step(const Dev& g, const SweepBufs& b, int num_sms, cudaStream_t s,
                         const cudaGraphConditionalHandle* cond);
+// The same loop in one cooperative launch (`start`: begin first, with these
+// host fields), as long as a
+// sweep visits at most kFusedMax vertices: b.rc->cont stays 1 for the kernels
+// above to go on where the next one visits more. With `cond`, that graph
+// conditional receives b.rc->cont.
+constexpr uint32_t kFusedMax = 1u << 19;
+void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start, int num_sms, cudaStream_t s,
+                         const cudaGraphConditionalHandle* cond);
 void launch_query(const uint16_t* snap, uint32_t n, const uint32_t* v, uint16_t* out, uint32_t k, cudaStream_t s);
 void launch_color_list(const Dev& g, const uint32_t* list, uint32_t m, uint32_t* colored, cudaStream_t s);
 void launch_snapshot_changes(const Dev& g, uint32_t* prev, uint16_t* snap, cudaStream_t s);

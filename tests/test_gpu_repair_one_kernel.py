@@ -1,0 +1,41 @@
+"""The repair as one kernel against the same passes as kernels of their own
+(which timed handles run), array by array, around the sizes where it goes from
+the whole grid to a few blocks and where it leaves a sweep to the others."""
+import numpy as np
+import pytest
+
+import streamgc_b200 as S
+
+pytestmark = pytest.mark.gpu
+
+
+def graph(n, seed):
+    """A ring with random chords and, where there is room, hub rows on both sides
+    of the per-thread limit (64 slots) and of one and two work items (512)."""
+    rng = np.random.default_rng(seed)
+    v = np.arange(n)
+    e = [np.stack([v, (v + 1) % n], 1), rng.integers(0, n, (n, 2))]
+    for k, deg in enumerate((64, 65, 511, 513, 5000)):
+        if deg < n // 2:
+            e.append(np.stack([np.full(deg, k), rng.choice(np.arange(8, n), deg, replace=False)], 1))
+    e = np.concatenate(e)
+    return S.Graph.from_edges(n, e[e[:, 0] != e[:, 1]])
+
+
+@pytest.mark.parametrize("exact", [True, False], ids=["exact", "reference"])
+@pytest.mark.parametrize("n", [3, 33, 2047, 2049, 40000, (1 << 19) - 1, (1 << 19) + 1])
+def test_same_as_the_separate_kernels(n, exact):
+    g = graph(n, n)
+    churn = g.churn_stream(min(2 * n, 20000), 50, 3)
+    with S.StreamGC(g, exact_select=exact, profile=True, full_repair_every=2) as a, \
+            S.StreamGC(g, exact_select=exact, full_repair_every=2) as b:
+        for k in range(4):  # from no color, then after updates: full and incremental repairs
+            ra, rb = a.publish(), b.publish()
+            assert ra == rb
+            for what in ("states", "bitmaps", "snapshot", "col"):
+                assert np.array_equal(getattr(a, what)(), getattr(b, what)()), (k, what)
+            sa, sb = a.stats(), b.stats()
+            assert sa["live_entries"] == sb["live_entries"] and sb["device_error"] == 0
+            part = churn[k * 4096:(k + 1) * 4096]
+            a.apply(part, S.MODE_DETERMINISTIC)
+            b.apply(part, S.MODE_DETERMINISTIC)
