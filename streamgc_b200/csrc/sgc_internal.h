@@ -78,6 +78,8 @@ struct sgc_handle {
     uint32_t* dirty_list = nullptr;
     sgc::Tier2Bufs t2{};
     uint32_t* h_small = nullptr;         // pinned readback scratch
+    uint32_t* query_v = nullptr;         // pinned, mapped: a query's vertices and colors (made on first use)
+    uint16_t* query_out = nullptr;
     sgc::RepairCtl* h_rc_in = nullptr;   // pinned: host fields of the repair control block
     sgc::RepairCtl* h_rc_out = nullptr;  // pinned: its readback
     uint64_t repairs_since_full = 0;
