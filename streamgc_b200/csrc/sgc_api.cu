@@ -1038,7 +1038,7 @@ int sgc_validate(sgc_handle* h, sgc_validation* out) {
     if (!h || !out) return fail(SGC_EINVAL, "null argument");
     CK(cudaSetDevice(h->device));
     uint64_t v[5] = {0, 0, 0, 0, 0};
-    const int r = run_validate(h->g, h->stream, v);
+    const int r = run_validate(h->g, reinterpret_cast<unsigned long long*>(h->t2.count), h->h_small, h->stream, v);
     if (r < 0) return fail(SGC_ECUDA, "validator failed (%d)", r);
     out->violations = v[0];
     out->uncolored_with_edges = v[1];

@@ -212,7 +212,8 @@ void launch_t2_span(const Dev& g, uint32_t G, uint32_t* span, cudaStream_t s);
 size_t tier2_cub_bytes(uint32_t n, uint32_t rev_cap);
 
 // Validator (sgc_tier2.cu): [violations, uncolored_with_edges, distinct_edges, max_color, out_of_range]
-int run_validate(const Dev& g, cudaStream_t s, uint64_t* out);
+// `words`: six words on the device, `host`: 48 bytes pinned.
+int run_validate(const Dev& g, unsigned long long* words, uint32_t* host, cudaStream_t s, uint64_t* out);
 // Layout invariants of every row: out = {rows breaking one, SGC_STATE_* bits
 // seen, lowest such row (~0 if none)}.
 int run_check_state(const Dev& g, cudaStream_t s, uint64_t* out);
