@@ -596,6 +596,7 @@ int sgci::create_internal(const StreamGCConfig* cfg, const sgc_options* opt_in, 
     A(&t2.rev_end, n);
     A(&t2.pend_v, n);
     A(&t2.pend_w, n);
+    A(&h->color_rows, kColorWords);
     t2.rev_cap = 1u << 20;
     if (cudaMalloc(&t2.rev_keys, (size_t)t2.rev_cap * 8) || cudaMalloc(&t2.rev_keys2, (size_t)t2.rev_cap * 8))
         return bail(fail(SGC_ENOMEM, "tier-2 reverse buffer allocation failed"));
@@ -1011,7 +1012,8 @@ int sgc_color_core(sgc_handle* h, uint32_t min_degree, uint32_t* colored) {
     if (!list.empty()) {
         uint32_t* d = h->t2.list;  // idle between repairs
         CK(cudaMemcpyAsync(d, list.data(), list.size() * 4, cudaMemcpyHostToDevice, h->stream));
-        launch_color_list(h->g, d, (uint32_t)list.size(), h->t2.count, h->stream);
+        launch_color_list(h->g, d, (uint32_t)list.size(), h->t2.rev_start, h->color_rows, h->sb.bar, h->t2.count,
+                          h->num_sms, h->stream);
         h->launches += 1;
         CK(cudaMemcpyAsync(h->h_small, h->t2.count, 4, cudaMemcpyDeviceToHost, h->stream));
         for (uint32_t k = 0; k < std::max<uint32_t>(h->sb.G, 1u); k++)  // every graph's next repair is full

@@ -77,6 +77,7 @@ struct sgc_handle {
     sgc::SweepBufs sb{};
     uint32_t* dirty_list = nullptr;
     sgc::Tier2Bufs t2{};
+    uint32_t* color_rows = nullptr;      // scratch of sgc_color_core
     uint32_t* h_small = nullptr;         // pinned readback scratch
     uint32_t* query_v = nullptr;         // pinned, mapped: a query's vertices and colors (made on first use)
     uint16_t* query_out = nullptr;

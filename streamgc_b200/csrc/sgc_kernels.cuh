@@ -171,7 +171,12 @@ constexpr uint32_t kFusedMax = 1u << 19;
 void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start, int num_sms, cudaStream_t s,
                          const cudaGraphConditionalHandle* cond);
 void launch_query(const uint16_t* snap, uint32_t n, const uint32_t* v, uint16_t* out, uint32_t k, cudaStream_t s);
-void launch_color_list(const Dev& g, const uint32_t* list, uint32_t m, uint32_t* colored, cudaStream_t s);
+// First-fit coloring of list[0, m) in list order. `place`: n words, `rows`:
+// kColorWords words of scratch; `colored` receives how many had no color.
+constexpr uint32_t kColorWindow = 128;  // vertices gathered at once
+constexpr uint32_t kColorWords = kColorWindow * (64 + kColorWindow / 32);
+void launch_color_list(const Dev& g, const uint32_t* list, uint32_t m, uint32_t* place, uint32_t* rows, GridBar* bar,
+                       uint32_t* colored, int num_sms, cudaStream_t s);
 void launch_snapshot_changes(const Dev& g, uint32_t* prev, uint16_t* snap, cudaStream_t s);
 void launch_colors(const Dev& g, uint16_t* out, cudaStream_t s);
 
