@@ -736,6 +736,9 @@ void launch_query(const uint16_t* snap, uint32_t n, const uint32_t* v, uint16_t*
 // sweeps over many vertices, and timed ones, run pass by pass as kernels of their
 // own, between which the host or a CUDA-graph while-node reads the decision.
 
+// Worklists short enough for a few blocks (see the one-kernel repair).
+constexpr uint32_t kTailBlocks = 16, kTailList = 2048, kTailItems = 768;
+
 // list_mode of the per-vertex passes: 0 every vertex, 1 b.wl, 2 as RepairCtl says.
 __device__ __forceinline__ bool use_list(const SweepBufs& b, int list_mode) {
     return list_mode == 2 ? ld_cg(&b.rc->list) != 0 : list_mode == 1;
@@ -1277,8 +1280,10 @@ __device__ __forceinline__ void collect_marks(const Dev& g, const SweepBufs& b, 
             if (bits) b.wmark[w] = 0;
         }
         list_bits(w, bits, b.wl, b.wl_count);
-        uint32_t k = 0;  // the work items they will make
-        for (uint32_t r = bits; r; r &= r - 1) {
+        // the work items they will make (asked for only of a short list: many marks
+        // in one word count as too many, and cost no walk over their rows)
+        uint32_t k = __popc(bits) > 4 ? 4 * kTailItems + 1 : 0u;
+        for (uint32_t r = k ? 0u : bits; r; r &= r - 1) {
             const uint32_t len = row_len(g, w * 32 + (__ffs(r) - 1));
             if (len > SWEEP_TINY) k += (len + b.tile - 1) / b.tile;
         }
@@ -1490,7 +1495,7 @@ void launch_repair_begin(const Dev& g, const SweepBufs& b, SweepMode mode, int n
 // sweep over many vertices, where the item passes' 40 warps per SM pay and a
 // launch costs little, is left to the kernels above.
 constexpr uint32_t kFusedThreads = 768;
-constexpr uint32_t kTailBlocks = 16, kTailList = 2048, kTailItems = 768;
+
 
 // The first `nb` blocks of the grid meet. A thread's writes before the barrier
 // are seen after it by plain loads in all of them. Round by round the arrivals
