@@ -92,15 +92,15 @@ int compact_dirty(sgc_handle* h, bool force) {
     CK(cudaMemsetAsync(&h->ctl->dirty_count, 0, 4, h->stream));
     launch_dirty_list(h->g, h->dirty_list, &h->ctl->dirty_count, h->stream);
     launch_compact(h->g, h->dirty_list, &h->ctl->dirty_count, h->n, force, h->stream,
-                   (h->opt.flags & SGC_OPT_SORTED_ROWS) != 0);
+                   (h->opt.flags & SGC_OPT_SORTED_ROWS) != 0, &h->ctl->drain_n);
     h->launches += 2;
     return check_cuda("compact");
 }
 
+// The overflow entries that the compaction before this took.
 int drain(sgc_handle* h, bool ordered, unsigned long long* failed_counter) {
-    launch_take_overflow(h->g, &h->ctl->drain_n, h->stream);
     launch_drain(h->g, &h->ctl->drain_n, ordered, failed_counter, h->stream);
-    h->launches += 2;
+    h->launches += 1;
     return check_cuda("drain");
 }
 

@@ -129,8 +129,8 @@ void enqueue_head(sgc_batch* b, cudaStream_t s, const cudaGraphConditionalHandle
     launch_add_check(h->g, h->d_batch, 0, b->d_dyn, h->num_sms, s);
     cudaMemsetAsync(&h->ctl->dirty_count, 0, 4, s);
     launch_dirty_list(h->g, h->dirty_list, &h->ctl->dirty_count, s);
-    launch_compact(h->g, h->dirty_list, &h->ctl->dirty_count, h->n, false, s, (h->opt.flags & SGC_OPT_SORTED_ROWS) != 0);
-    launch_take_overflow(h->g, &h->ctl->drain_n, s);
+    launch_compact(h->g, h->dirty_list, &h->ctl->dirty_count, h->n, false, s, (h->opt.flags & SGC_OPT_SORTED_ROWS) != 0,
+                   &h->ctl->drain_n);
     launch_drain(h->g, &h->ctl->drain_n, (b->flags & SGC_BATCH_STREAM_ORDER) != 0, &h->ctl->drain_failed, s);
     const RepairIn in{(uint32_t)SWEEP_INDEP, 64u, 0u};
     launch_repair_fused(h->g, h->sb, &in, h->num_sms, s, cond);

@@ -15,7 +15,7 @@
 //                         of only the rows edited since their last compaction
 //                         (every other row is already compact, so compacting it
 //                         is the identity); reads each row up to its high-water.
-//   take_overflow/drain   streamgc.cu:967-995 + epoch_maintenance.cu:66-87.
+//   drain                 streamgc.cu:967-995 + epoch_maintenance.cu:66-87.
 //   sweep                 degree-balanced pass over every live adjacency entry:
 //                         rebuild_bitmaps (epoch_maintenance.cu:113-128) and the
 //                         Tier-1 decision (conflict_repair.cu:10-114) fused, as a
@@ -534,100 +534,114 @@ __device__ __forceinline__ void warp_sort_row(uint32_t* buf, uint32_t m, uint32_
         }
 }
 
+// A lane decides about a row of its own, so the words of 32 rows arrive in one
+// round; the warp then compacts, one after another, those that need it. (A warp
+// per row spent two round trips on each row it left alone: 16 us for the 50,000
+// rows of an epoch of 32,768 updates on a mesh, 67 us for 262,144 on a power-law
+// graph; now 8 and 30.) One thread takes the overflow count for the drain that
+// follows (`drain_n` non-null); nothing appends to the buffer meanwhile.
 __global__ void __launch_bounds__(256) compact_kernel(Dev g, const uint32_t* __restrict__ list,
-                                                      const uint32_t* __restrict__ count, int force, int merge) {
+                                                      const uint32_t* __restrict__ count, int force, int merge,
+                                                      uint32_t* drain_n) {
     extern __shared__ uint32_t sort_buf[];  // kMergeMax words per warp, only with `merge`
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t lane = lane_id();
     const uint32_t cnt = *count;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const uint32_t c = *g.ovf_count;
+        if (c) *g.ovf_count = 0;
+        *drain_n = c < OVF_CAP ? c : OVF_CAP;
+    }
     merge = merge && g.blen;
-    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < cnt; k += warps) {
-        const uint32_t x = list[k];
-        const uint64_t s = g.rp[x];
-        const uint32_t hwx = row_len(g, x);
-        // Lazy mode: a row whose holes fill at most a quarter of its extent stays
-        // as it is (every reader skips INV slots and tombstones); it is compacted later.
-        const uint32_t run = merge ? min(g.blen[x], hwx) : 0u;
-        const bool long_tail = merge && hwx - run > max(32u, hwx >> 3);
-        const uint32_t holes = g.live ? row_holes(g, x, g.hw[x]) : 0u;
-        if (!force && g.live && 4u * holes <= hwx && !long_tail) {
-            if ((holes || (merge && run < hwx)) && lane == 0)  // still a candidate (holes, or a tail to merge)
-                atomicOr(g.dirty + (x >> 5), 1u << (x & 31));
-            continue;
+    // as many rows per warp as leave every warp something to do
+    const uint32_t each = cnt >= 32 * warps ? 32u : (cnt + warps - 1) / warps;
+    for (uint32_t k0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * each; k0 < cnt; k0 += warps * each) {
+        uint32_t row = 0, row_hw = 0, row_run = 0;
+        uint64_t row_s = 0;
+        bool todo = false;
+        if (lane < each && k0 + lane < cnt) {
+            row = list[k0 + lane];
+            row_s = g.rp[row];
+            row_hw = row_len(g, row);
+            row_run = g.blen ? g.blen[row] : 0u;
+            // Lazy mode: a row whose holes fill at most a quarter of its extent stays
+            // as it is (every reader skips INV slots and tombstones); it is compacted later.
+            const uint32_t run = merge ? min(row_run, row_hw) : 0u;
+            const bool long_tail = merge && row_hw - run > max(32u, row_hw >> 3);
+            const uint32_t holes = g.live ? row_holes(g, row, g.hw[row]) : 0u;
+            todo = force || !g.live || 4u * holes > row_hw || long_tail;
+            if (!todo && (holes || (merge && run < row_hw)))  // still a candidate (holes, or a tail to merge)
+                atomicOr(g.dirty + (row >> 5), 1u << (row & 31));
         }
-        const uint64_t e = s + hwx;
-        const uint64_t run_end = s + (g.blen ? g.blen[x] : 0u);
-        uint64_t w = s, run_live = 0;
-        for (uint64_t c = s & ~3ull; c < e; c += 128) {
-            const uint64_t i = c + 4ull * lane;
-            uint4 q = make_uint4(INV, INV, INV, INV);
-            if (i < e) q = ld_cg4(g.col + i);
-            uint32_t vals[4] = {q.x, q.y, q.z, q.w};
-            uint32_t m = 0, mr = 0;
+        for (uint32_t left = __ballot_sync(FULL, todo); left; left &= left - 1) {
+            const int src = __ffs(left) - 1;
+            const uint32_t x = __shfl_sync(FULL, row, src), hwx = __shfl_sync(FULL, row_hw, src);
+            const uint64_t s = __shfl_sync(FULL, (unsigned long long)row_s, src);
+            const uint64_t e = s + hwx;
+            const uint64_t run_end = s + __shfl_sync(FULL, row_run, src);
+            uint64_t w = s, run_live = 0;
+            for (uint64_t c = s & ~3ull; c < e; c += 128) {
+                const uint64_t i = c + 4ull * lane;
+                uint4 q = make_uint4(INV, INV, INV, INV);
+                if (i < e) q = ld_cg4(g.col + i);
+                uint32_t vals[4] = {q.x, q.y, q.z, q.w};
+                uint32_t m = 0, mr = 0;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const bool live = g.blen ? (vals[j] & TOMB) == 0 : vals[j] != INV;
-                if (i + j >= s && i + j < e && live) {
-                    m |= 1u << j;
-                    if (i + j < run_end) mr |= 1u << j;
+                for (int j = 0; j < 4; j++) {
+                    const bool live = g.blen ? (vals[j] & TOMB) == 0 : vals[j] != INV;
+                    if (i + j >= s && i + j < e && live) {
+                        m |= 1u << j;
+                        if (i + j < run_end) mr |= 1u << j;
+                    }
                 }
+                run_live += __reduce_add_sync(FULL, (uint32_t)__popc(mr));
+                uint32_t total = 0;
+                const uint32_t pre = warp_excl_scan(__popc(m), total);
+                __syncwarp();
+                uint64_t dst = w + pre;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (m & (1u << j)) {
+                        if (dst != i + j) g.col[dst] = vals[j];
+                        dst++;
+                    }
+                w += total;
+                __syncwarp();
             }
-            run_live += __reduce_add_sync(FULL, (uint32_t)__popc(mr));
-            uint32_t total = 0;
-            const uint32_t pre = warp_excl_scan(__popc(m), total);
-            __syncwarp();
-            uint64_t dst = w + pre;
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                if (m & (1u << j)) {
-                    if (dst != i + j) g.col[dst] = vals[j];
-                    dst++;
-                }
-            w += total;
+            for (uint64_t j = w + lane; j < e; j += 32) g.col[j] = INV;
+            const uint32_t live = (uint32_t)(w - s);
+            if (merge && live > run_live && live <= kMergeMax) {  // tail entries behind the run: one sorted run
+                __syncwarp();
+                uint32_t* buf = sort_buf + ((threadIdx.x >> 5) & 7) * kMergeMax;
+                const uint32_t m = live < 2 ? live : 1u << (32 - __clz(live - 1));
+                for (uint32_t i = lane; i < m; i += 32) buf[i] = i < live ? g.col[s + i] : INV;
+                __syncwarp();
+                warp_sort_row(buf, m, lane);
+                for (uint32_t i = lane; i < live; i += 32) g.col[s + i] = buf[i];
+                run_live = live;
+            }
+            if (lane == 0) {
+                g.hw[x] = live;
+                if (g.live) g.live[x] = live;
+                if (g.blen) g.blen[x] = (uint32_t)run_live;
+            }
             __syncwarp();
         }
-        for (uint64_t j = w + lane; j < e; j += 32) g.col[j] = INV;
-        const uint32_t live = (uint32_t)(w - s);
-        if (merge && live > run_live && live <= kMergeMax) {  // tail entries behind the run: one sorted run
-            __syncwarp();
-            uint32_t* buf = sort_buf + ((threadIdx.x >> 5) & 7) * kMergeMax;
-            const uint32_t m = live < 2 ? live : 1u << (32 - __clz(live - 1));
-            for (uint32_t i = lane; i < m; i += 32) buf[i] = i < live ? g.col[s + i] : INV;
-            __syncwarp();
-            warp_sort_row(buf, m, lane);
-            for (uint32_t i = lane; i < live; i += 32) g.col[s + i] = buf[i];
-            run_live = live;
-        }
-        if (lane == 0) {
-            g.hw[x] = live;
-            if (g.live) g.live[x] = live;
-            if (g.blen) g.blen[x] = (uint32_t)run_live;
-        }
-        __syncwarp();
     }
 }
 
 void launch_compact(const Dev& g, const uint32_t* list, const uint32_t* count, uint32_t max_rows, bool force,
-                    cudaStream_t s, bool merge) {
-    if (!max_rows) return;
+                    cudaStream_t s, bool merge, uint32_t* drain_n) {
     uint32_t blocks = (max_rows + 7) / 8;
     if (blocks > 148 * 16) blocks = 148 * 16;
     const size_t smem = merge && g.blen ? 8 * kMergeMax * sizeof(uint32_t) : 0;  // 32 KiB: under the 48 KiB default
-    compact_kernel<<<blocks, 256, smem, s>>>(g, list, count, force ? 1 : 0, (merge && g.blen) ? 1 : 0);
+    compact_kernel<<<blocks, 256, smem, s>>>(g, list, count, force ? 1 : 0, (merge && g.blen) ? 1 : 0,
+                                         drain_n);
 }
 
 // ---------------------------------------------------------------------------
 // overflow drain (streamgc.cu:967-995, epoch_maintenance.cu:66-87)
 // ---------------------------------------------------------------------------
-
-__global__ void take_overflow_kernel(Dev g, uint32_t* drain_n) {
-    const uint32_t c = *g.ovf_count;
-    if (c) *g.ovf_count = 0;
-    *drain_n = c < OVF_CAP ? c : OVF_CAP;
-}
-void launch_take_overflow(const Dev& g, uint32_t* drain_n, cudaStream_t s) {
-    take_overflow_kernel<<<1, 1, 0, s>>>(g, drain_n);
-}
 
 // Re-insert without re-appending: first INV or equal slot; none -> failure.
 // Unordered drains under exact selection look in the sorted base run first.

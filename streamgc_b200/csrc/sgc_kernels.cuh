@@ -131,10 +131,10 @@ void launch_seg_apply(const Dev& g, const EdgeUpdate* ups, const uint32_t* segs,
                       int num_sms, cudaStream_t s);
 void launch_dirty_list(const Dev& g, uint32_t* list, uint32_t* count, cudaStream_t s);
 // force: compact every listed row (else rows whose holes fill at most a quarter
-// of their extent wait, under exact selection).
+// of their extent wait, under exact selection). *drain_n receives the number of
+// overflow entries to drain; their count starts again at 0.
 void launch_compact(const Dev& g, const uint32_t* list, const uint32_t* count, uint32_t max_rows, bool force,
-                    cudaStream_t s, bool merge = false);
-void launch_take_overflow(const Dev& g, uint32_t* drain_n, cudaStream_t s);
+                    cudaStream_t s, bool merge, uint32_t* drain_n);
 void launch_drain(const Dev& g, const uint32_t* drain_n, bool ordered, unsigned long long* failed, cudaStream_t s);
 void launch_snapshot(const Dev& g, uint16_t* snap, cudaStream_t s);
 // list_mode 0: every vertex; 1: the vertices in b.wl; 2: as b.rc->list says.
