@@ -696,36 +696,30 @@ __device__ __forceinline__ void new_nbr(const Dev& g, uint32_t x, uint16_t c) {
 // ---------------- recolor (recolor.cu:87-163) ----------------
 
 // Concurrent batches: the change of a neighbor's color old -> new walked to
-// every live entry of [s, e). A lane reads eight entries and their bitmaps
+// every live entry of [s, e). A lane reads four entries and their bitmaps
 // before it sets a bit.
 __device__ __forceinline__ void warp_walk(const Dev& g, uint64_t s, uint64_t e, uint16_t oldc, uint16_t newc) {
     const uint32_t lane = lane_id();
     const uint64_t bit = newc != 0 && newc <= 64 ? 1ull << (newc - 1) : 0ull;
     if (g.exact && !bit) return;
 #pragma unroll 1
-    for (uint64_t c = s & ~3ull; c < e; c += 256) {
-        const uint64_t i0 = c + 4ull * lane, i1 = i0 + 128;
-        uint4 q0 = make_uint4(INV, INV, INV, INV), q1 = q0;
-        if (i0 < e) q0 = ld_cg4(g.col + i0);
-        if (i1 < e) q1 = ld_cg4(g.col + i1);
-        uint32_t y[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        uint64_t bm[8];
+    for (uint64_t c = s & ~3ull; c < e; c += 128) {
+        const uint64_t i = c + 4ull * lane;
+        uint4 q = make_uint4(INV, INV, INV, INV);
+        if (i < e) q = ld_cg4(g.col + i);
+        const uint32_t y[4] = {q.x, q.y, q.z, q.w};
+        uint64_t bm[4];
+        bool in[4];
 #pragma unroll
-        for (int t = 0; t < 8; t++) {
-            const uint64_t p = (t < 4 ? i0 : i1) + (t & 3);
-            if (!(p >= s && p < e && y[t] < g.n)) y[t] = INV;
-            bm[t] = y[t] != INV && bit ? ld_cg(g.bm + y[t]) : ~0ull;
+        for (int t = 0; t < 4; t++) {
+            in[t] = i + t >= s && i + t < e && y[t] < g.n;
+            bm[t] = in[t] && bit ? ld_cg(g.bm + y[t]) : ~0ull;
         }
 #pragma unroll
-        for (int t = 0; t < 8; t++)
+        for (int t = 0; t < 4; t++) {
             if (bit & ~bm[t]) atomicOr((unsigned long long*)(g.bm + y[t]), (unsigned long long)bit);
-        if (g.exact) continue;
-#pragma unroll 1
-        for (int t = 0; t < 8; t++) {
-            uint32_t z = INV;  // y[t], by selects: the array stays in registers
-#pragma unroll
-            for (int k = 0; k < 8; k++) z = k == t ? y[k] : z;
-            const uint32_t hd = z != INV ? __ldg(g.hdmap + z) : EMPTY;
+            if (g.exact || !in[t]) continue;
+            const uint32_t hd = __ldg(g.hdmap + y[t]);
             if (hd == EMPTY) continue;
             uint32_t* h = g.hist + (uint64_t)hd * g.maxc;
             if (oldc != 0 && oldc <= g.maxc) atomicSub(h + oldc - 1, 1u);
