@@ -343,6 +343,9 @@ __device__ __forceinline__ void flag_asym(const Dev& g, uint32_t x) {
     uint32_t* a = &g.gctl[graph_of(g, x)].asym;
     if (!ld_cg(a)) atomicOr(a, 1u);
 }
+__device__ __forceinline__ bool pristine(const Dev& g, uint32_t x) {
+    return !(ld_cg(g.edited + (x >> 5)) & (1u << (x & 31)));
+}
 
 // Group-collective W-ary search for `key` in the ascending run col[s, e):
 // each round probes W evenly spaced slots and keeps the bucket holding the
@@ -367,31 +370,81 @@ __device__ __forceinline__ uint64_t grp_bsearch(const Lanes<W>& L, const uint32_
     return b ? lo + (__ffs(b) - 1) : ~0ull;
 }
 
-// W-ary search by id in a sorted run (ascending ids; with `tomb` a deleted
-// entry keeps its id under that bit). Returns the slot index, or ~0 when the id
-// is absent; `val` gets the slot's value (the id, or id | tomb).
+// W-ary search by id in a base run (ascending ids, tombstones keep their id
+// under TOMB). Returns the slot index, or ~0 when the id is absent; `val` gets
+// the slot's value (the id, or id | TOMB).
 template <int W>
 __device__ __forceinline__ uint64_t grp_bsearch_key(const Lanes<W>& L, const uint32_t* col, uint64_t s, uint64_t e,
-                                                    uint32_t key, uint32_t tomb, uint32_t& val) {
-    uint64_t lo = s;
-    uint32_t len = (uint32_t)(e - s);
-    while (len > W) {
-        const uint32_t step = len / W;
-        const uint32_t v = ld_cg(col + lo + L.lane * step) & ~tomb;
+                                                    uint32_t key, uint32_t& val) {
+    uint64_t lo = s, hi = e;
+    while (hi - lo > W) {
+        const uint64_t step = (hi - lo) / W;
+        const uint32_t v = ld_cg(col + lo + L.lane * step) & ~TOMB;
         const uint32_t b = L.ballot(v <= key);
         if (!b) return ~0ull;
         const uint32_t top = 31 - __clz(b);
-        lo += top * step;
-        len = top == W - 1 ? len - top * step : step;
+        const uint64_t nlo = lo + top * step;
+        hi = (top == W - 1) ? hi : nlo + step;
+        lo = nlo;
     }
-    const uint32_t v = L.lane < len ? ld_cg(col + lo + L.lane) : INV;
-    const uint32_t b = L.ballot(L.lane < len && (v & ~tomb) == key);
+    const uint64_t i = lo + L.lane;
+    const uint32_t v = i < hi ? ld_cg(col + i) : INV;
+    const uint32_t b = L.ballot(i < hi && (v & ~TOMB) == key);
     if (!b) return ~0ull;
     val = L.shfl(v, __ffs(b) - 1);
     return lo + (__ffs(b) - 1);
 }
 
 // ---------------- slack-CSR row edits (local_update.cu:12-56) ----------------
+
+enum { ADD_INSERTED = 0, ADD_PRESENT = 1, ADD_OVERFLOW = 2 };
+
+// Concurrent batches under exact selection: rows keep their base run sorted
+// (a delete there leaves a tombstone, a re-insert of the same id revives it),
+// so an update finds a base entry by a W-ary search; only entries inserted
+// since the row's last compaction (its tail) are scanned. The updates of one
+// edge are ordered, so no other warp touches the slot of `nbr` meanwhile.
+// Add: returns ADD_PRESENT / ADD_INSERTED when the run holds nbr (live or
+// tombstone), -1 when it does not.
+template <int W>
+__device__ __forceinline__ int grp_run_add(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr, uint64_t s,
+                                           uint32_t bl) {
+    uint32_t val = 0;
+    const uint64_t p = grp_bsearch_key(L, g.col, s, s + bl, nbr, val);
+    if (p == ~0ull) return -1;
+    if (val == nbr) return ADD_PRESENT;
+    uint32_t old = 0;
+    if (L.leader()) {
+        old = atomicCAS(g.col + p, nbr | TOMB, nbr);
+        if (old == (nbr | TOMB)) {
+            atomicAdd(g.live + x, 1u);
+            mark_dirty(g, x);
+        }
+    }
+    old = L.shfl(old, 0);
+    return old == nbr ? ADD_PRESENT : ADD_INSERTED;
+}
+__device__ __forceinline__ int warp_run_add(const Dev& g, uint32_t x, uint32_t nbr, uint64_t s, uint32_t bl) {
+    return grp_run_add(Lanes<32>(), g, x, nbr, s, bl);
+}
+// Delete: true when the run held nbr live (now a tombstone).
+template <int W>
+__device__ __forceinline__ bool grp_run_remove(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr, uint64_t s,
+                                               uint32_t bl) {
+    uint32_t val = 0;
+    const uint64_t p = grp_bsearch_key(L, g.col, s, s + bl, nbr, val);
+    if (p == ~0ull || val != nbr) return false;
+    uint32_t old = 0;
+    if (L.leader()) {
+        old = atomicCAS(g.col + p, nbr, nbr | TOMB);
+        if (old == nbr) {
+            atomicSub(g.live + x, 1u);
+            mark_dirty(g, x);
+        }
+    }
+    old = L.shfl(old, 0);
+    return old == nbr;
+}
 
 // A row without a free slot (one lane): the entry goes to the overflow buffer
 // (the counter always advances, the entry is stored only below capacity); the
@@ -412,131 +465,115 @@ __device__ __forceinline__ void append_overflow(const Dev& g, uint32_t x, uint32
     flag_asym(g, x);
 }
 
-// Group-collective: the first slot p in [s, e) that holds `nbr` or, with `free`,
-// nothing; two 16-byte loads per lane in flight.
+// add_local_neighbor: claim the first INV slot unless `nbr` shows up first;
+// a full row appends to the overflow buffer. The row's bounds, base run and high-water
+// mark are read together up front (a mark read early is only lower: the
+// fallback scan to the row's end covers what it misses).
 template <int W>
-__device__ __forceinline__ bool grp_find_slot(const Lanes<W>& L, const uint32_t* col, uint64_t s, uint64_t e,
-                                              uint32_t nbr, bool free, uint64_t& pos, uint32_t& val) {
-    constexpr uint64_t R = 4ull * W;
-    const uint32_t other = free ? INV : nbr;
-    for (uint64_t c = s & ~3ull; c < e; c += 2 * R) {
-        const uint64_t i0 = c + 4ull * L.lane, i1 = i0 + R;
-        uint4 q0 = make_uint4(0, 0, 0, 0), q1 = q0;
-        if (i0 < e) q0 = ld_cg4(col + i0);
-        if (i1 < e) q1 = ld_cg4(col + i1);
-        const auto pred = [nbr, other](uint32_t t) { return t == nbr || t == other; };
-        const uint32_t m0 = i0 < e ? mask4(q0, i0, s, e, pred) : 0u, m1 = i1 < e ? mask4(q1, i1, s, e, pred) : 0u;
-        uint32_t b = L.ballot(m0 != 0);
-        const bool first = b != 0;
-        if (!first) b = L.ballot(m1 != 0);
-        if (b) {
-            const int src = __ffs(b) - 1, kk = __ffs(first ? m0 : m1) - 1;
-            const uint32_t v = (first ? m0 : m1) ? pick4(first ? q0 : q1, kk) : 0u;
-            pos = c + (first ? 0ull : R) + 4ull * src + L.shfl(kk, src);
-            val = L.shfl(v, src);
-            return true;
+__device__ __forceinline__ int grp_add_slot(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr) {
+    const uint64_t s = g.rp[x], e = g.rp[x + 1];
+    const uint32_t bl = g.blen ? ld_cg(g.blen + x) : 0u;
+    const uint32_t hw0 = ld_cg(g.hw + x);
+    uint64_t from = s;
+    if (g.blen) {
+        if (bl) {
+            const int r = grp_run_add(L, g, x, nbr, s, bl);
+            if (r >= 0) return r;
         }
+        from = s + bl;  // the tail: first INV or nbr
+    } else if (pristine(g, x)) {
+        // Sorted base entries, no holes: the scan would stop at nbr if present,
+        // else at the first INV right after the base run.
+        const uint64_t len = live_end(g, x, s) - s;
+        if (grp_bsearch(L, g.col, s, s + len, nbr) != ~0ull) return ADD_PRESENT;
+        // Past the sorted run: the updates of this edge are ordered, so nbr can
+        // only be in the row through an earlier update of the edge, and that
+        // one would have marked the row edited.
+        from = s + len;
     }
-    return false;
-}
-
-enum { ADD_INSERTED = 0, ADD_PRESENT = 1, ADD_OVERFLOW = 2 };
-
-// One row edit of a concurrent batch (add_local_neighbor, remove_local_neighbor;
-// local_update.cu:12-56): row x gets or loses `nbr`. One function for both, so
-// that the update path holds one copy of each search.
-//   Add: the first free slot is claimed unless `nbr` shows up first; a full row
-// appends to the overflow buffer. ADD_INSERTED / ADD_PRESENT / ADD_OVERFLOW.
-//   Remove: the first slot equal to `nbr` is freed. ADD_PRESENT when it was
-// there, else ADD_INSERTED.
-// Under exact selection rows keep their base run [0, blen) sorted: a delete
-// there leaves a tombstone, a re-insert of the same id revives it; only the
-// entries inserted since the row's last compaction (its tail) are scanned. The
-// updates of one edge are ordered, so no other warp touches the slot of `nbr`
-// meanwhile. Under the reference's rules a row never edited is such a run,
-// without tombstones. The row's bounds, run and mark are read together up front
-// (a mark read early is only lower: the scan to the row's end covers what it
-// misses).
-template <int W>
-__device__ __forceinline__ int grp_edit_row(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr, bool add) {
-    const uint64_t s = g.rp[x], cap = g.rp[x + 1];
-    const bool runs = g.blen != nullptr;
-    const uint32_t* bw = runs ? g.blen + x : g.edited + (x >> 5);
-    const uint32_t hw0 = ld_cg(g.hw + x), b0 = ld_cg(bw);
-    uint64_t top = s + hw0;
-    if (top > cap) {
-        if (L.leader()) atomicOr(g.err, ERR_ROW);
-        top = cap;
-    }
-    const uint32_t tomb = runs ? TOMB : 0u;
-    uint32_t bl = runs ? b0 : ((b0 >> (x & 31)) & 1u ? 0u : (uint32_t)(top - s));
-    if (bl > (uint32_t)(cap - s)) bl = (uint32_t)(cap - s);
-    uint64_t p = ~0ull;
-    uint32_t val = 0;
-    if (bl) p = grp_bsearch_key(L, g.col, s, s + bl, nbr, tomb, val);
-    // Past the run: under the reference's rules a delete looks through the whole
-    // row again (a concurrent edit may have misled the search); an insert goes
-    // on behind the sorted entries, where nbr can only be through an earlier
-    // update of the edge, which would have marked the row edited.
-    uint64_t from = (runs || add) ? s + bl : s;
-    // The first free slot at or after `from` lies at or below the mark, so an
-    // insert's first scan stops one slot past it; if a concurrent insert took
-    // those slots meanwhile, it goes on to the end of the row.
-    uint64_t lim = add ? (top < cap ? top + 1 : cap) : top;
-    bool in_run = p != ~0ull;
+    // The first free slot at or after `from` lies at or below the high-water
+    // mark, so the first scan stops one slot past it (not at the end of the
+    // row's slack); if a concurrent insert took those slots meanwhile, the
+    // scan goes on to the end of the row.
+    uint64_t lim = s + hw0 + 1;
+    if (lim > e) lim = e;
     for (;;) {
-        if (!in_run) {
-            const bool hit = from < lim && grp_find_slot(L, g.col, from, lim, nbr, add, p, val);
-            if (!hit) {
-                if (!add) return ADD_INSERTED;
-                if (lim < cap) {
-                    if (lim > from) from = lim;
-                    lim = cap;
-                    continue;
-                }
-                if (L.leader()) append_overflow(g, x, nbr);
-                L.sync();
-                return ADD_OVERFLOW;
-            }
-        }
-        // the slot's value now, and what the edit makes of it
-        const bool run_edit = in_run && runs;
-        if (add && val == nbr) return ADD_PRESENT;
-        if (!add && val != nbr) {  // a tombstone: not live in the run; the tail
-            in_run = false;
+        uint64_t p = 0;
+        uint32_t v = 0;
+        const bool hit =
+            from < lim && grp_find(L, g.col, from, lim, [nbr](uint32_t t) { return t == INV || t == nbr; }, p, v);
+        if (!hit && lim < e) {
+            if (lim > from) from = lim;
+            lim = e;
             continue;
         }
-        const uint32_t want = add ? nbr : (run_edit ? nbr | TOMB : INV);
+        if (!hit) {
+            if (L.leader()) append_overflow(g, x, nbr);
+            L.sync();
+            return ADD_OVERFLOW;
+        }
+        if (v == nbr) return ADD_PRESENT;
         uint32_t old = 0;
         if (L.leader()) {
-            old = atomicCAS(g.col + p, val, want);
-            if (old == val) {
-                if (add && !run_edit) atomicMax(g.hw + x, (uint32_t)(p - s) + 1);
-                if (g.live) atomicAdd(g.live + x, add ? 1u : ~0u);
-                if (!add && !run_edit && runs && p < s + ld_cg(g.blen + x)) g.blen[x] = 0;  // an INV inside the run ends it
+            old = atomicCAS(g.col + p, INV, nbr);
+            if (old == INV) {
+                extend_row(g, x, (uint32_t)(p - s));
                 mark_dirty(g, x);
             }
         }
         old = L.shfl(old, 0);
-        if (old == val) return add ? ADD_INSERTED : ADD_PRESENT;
-        if (add && old == nbr) return ADD_PRESENT;
-        if (add && run_edit) return ADD_INSERTED;
-        if (!in_run) from = p + 1;  // lost the slot to a concurrent edit: keep scanning after it
-        in_run = false;
+        if (old == INV) return ADD_INSERTED;
+        if (old == nbr) return ADD_PRESENT;
+        from = p + 1;  // lost the slot to a concurrent insert: keep scanning after it
     }
 }
+__device__ __forceinline__ int warp_add_slot(const Dev& g, uint32_t x, uint32_t nbr) {
+    return grp_add_slot(Lanes<32>(), g, x, nbr);
+}
 
-// Adds `nbr` to row x's base run when the run holds it, live or deleted (the drain).
-__device__ __forceinline__ bool warp_run_add(const Dev& g, uint32_t x, uint32_t nbr, uint64_t s, uint32_t bl) {
-    uint32_t val = 0;
-    const uint64_t p = grp_bsearch_key(Lanes<32>(), g.col, s, s + bl, nbr, TOMB, val);
-    if (p == ~0ull) return false;
-    if (val != nbr && lane_id() == 0 && atomicCAS(g.col + p, nbr | TOMB, nbr) == (nbr | TOMB)) {
-        atomicAdd(g.live + x, 1u);
-        mark_dirty(g, x);
+// remove_local_neighbor: first slot equal to nbr becomes INV (lazy delete).
+// Returns whether an entry was removed.
+template <int W>
+__device__ __forceinline__ bool grp_remove_slot(const Lanes<W>& L, const Dev& g, uint32_t x, uint32_t nbr) {
+    const uint64_t s = g.rp[x];
+    const uint32_t bl = g.blen ? ld_cg(g.blen + x) : 0u;
+    const uint64_t e = live_end(g, x, s);
+    uint64_t from = s;
+    if (g.blen) {
+        if (bl && grp_run_remove(L, g, x, nbr, s, bl)) return true;
+        from = s + bl;  // not live in the run: the tail
+    } else if (pristine(g, x)) {
+        const uint64_t p = grp_bsearch(L, g.col, s, e, nbr);
+        if (p != ~0ull) {
+            uint32_t old = 0;
+            if (L.leader()) {
+                old = atomicCAS(g.col + p, nbr, INV);
+                if (old == nbr) mark_dirty(g, x);
+            }
+            old = L.shfl(old, 0);
+            if (old == nbr) return true;
+        }
     }
-    __syncwarp();
-    return true;
+    for (;;) {
+        uint64_t p = 0;
+        uint32_t v = 0;
+        if (!grp_find(L, g.col, from, e, [nbr](uint32_t t) { return t == nbr; }, p, v)) return false;
+        uint32_t old = 0;
+        if (L.leader()) {
+            old = atomicCAS(g.col + p, nbr, INV);
+            if (old == nbr) {
+                mark_dirty(g, x);
+                if (g.live) atomicSub(g.live + x, 1u);
+                if (g.blen && p < s + ld_cg(g.blen + x)) g.blen[x] = 0;  // an INV inside the run ends it
+            }
+        }
+        old = L.shfl(old, 0);
+        if (old == nbr) return true;
+        from = p + 1;
+    }
+}
+__device__ __forceinline__ bool warp_remove_slot(const Dev& g, uint32_t x, uint32_t nbr) {
+    return grp_remove_slot(Lanes<32>(), g, x, nbr);
 }
 
 // ---------------- color selection (color_select.cuh:10-115) ----------------
@@ -693,46 +730,75 @@ __device__ __forceinline__ void new_nbr(const Dev& g, uint32_t x, uint16_t c) {
     const uint32_t hd = __ldg(g.hdmap + x);
     if (hd != EMPTY && !g.exact && c <= g.maxc) atomicAdd(g.hist + (uint64_t)hd * g.maxc + c - 1, 1u);
 }
-// ---------------- recolor (recolor.cu:87-163) ----------------
-
-// Concurrent batches: the change of a neighbor's color old -> new walked to
-// every live entry of [s, e). A lane reads four entries and their bitmaps
-// before it sets a bit.
-__device__ __forceinline__ void warp_walk(const Dev& g, uint64_t s, uint64_t e, uint16_t oldc, uint16_t newc) {
-    const uint32_t lane = lane_id();
-    const uint64_t bit = newc != 0 && newc <= 64 ? 1ull << (newc - 1) : 0ull;
-    if (g.exact && !bit) return;
-#pragma unroll 1
-    for (uint64_t c = s & ~3ull; c < e; c += 128) {
-        const uint64_t i = c + 4ull * lane;
-        uint4 q = make_uint4(INV, INV, INV, INV);
-        if (i < e) q = ld_cg4(g.col + i);
-        const uint32_t y[4] = {q.x, q.y, q.z, q.w};
-        uint64_t bm[4];
-        bool in[4];
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-            in[t] = i + t >= s && i + t < e && y[t] < g.n;
-            bm[t] = in[t] && bit ? ld_cg(g.bm + y[t]) : ~0ull;
-        }
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-            if (bit & ~bm[t]) atomicOr((unsigned long long*)(g.bm + y[t]), (unsigned long long)bit);
-            if (g.exact || !in[t]) continue;
-            const uint32_t hd = __ldg(g.hdmap + y[t]);
-            if (hd == EMPTY) continue;
-            uint32_t* h = g.hist + (uint64_t)hd * g.maxc;
-            if (oldc != 0 && oldc <= g.maxc) atomicSub(h + oldc - 1, 1u);
-            if (newc != 0 && newc <= g.maxc) atomicAdd(h + newc - 1, 1u);
-        }
-    }
-    __syncwarp();
+__device__ __forceinline__ void removed_nbr(const Dev& g, uint32_t x, uint16_t c) {
+    if (c == 0) return;
+    const uint32_t hd = __ldg(g.hdmap + x);
+    if (hd != EMPTY && !g.exact && c <= g.maxc) atomicSub(g.hist + (uint64_t)hd * g.maxc + c - 1, 1u);
 }
 
-// Does a live neighbor of x in [s, e) hold color c? Stops at the first round
-// that finds one.
-__device__ __forceinline__ bool warp_color_held(const Dev& g, uint64_t s, uint64_t e, uint16_t c) {
-    return warp_gather_each<true, 2>(g.col, s, e, g.n, g.st, [c](uint32_t, uint32_t w) { return color_of(w) == c; });
+// ---------------- recolor (recolor.cu:87-163) ----------------
+
+__device__ __forceinline__ uint32_t warp_load_state(const Dev& g, uint32_t x) {
+    uint32_t w = 0;
+    if (lane_id() == 0) w = ld_cg(g.st + x);
+    return __shfl_sync(FULL, w, 0);
+}
+
+// recolor_vertex: new = FAC(x); if different, CAS (new, version+1) in, retrying
+// on a fresh word; the winner propagates old -> new to every live row entry.
+// `chosen` (nonzero) is FAC(x) already computed on the current state by the
+// caller; in stream order nothing changes in between, so it equals the call
+// the reference makes here.
+// warp_recolor_from: the same with x's state word `cur` as last read by the
+// caller (a stale word fails the first compare-and-swap, which re-reads it).
+__device__ __forceinline__ void warp_recolor_from(const Dev& g, uint32_t x, uint16_t chosen, uint32_t cur) {
+    uint16_t newc = chosen ? chosen : warp_fac(g, x, g.st);
+    if (newc == color_of(cur)) return;
+    for (uint32_t tries = 0;; tries++) {
+        const uint32_t want = pack(newc, (uint16_t)(version_of(cur) + 1));
+        uint32_t got = 0;
+        if (lane_id() == 0) got = atomicCAS(g.st + x, cur, want);
+        got = __shfl_sync(FULL, got, 0);
+        if (got == cur) break;
+        if (tries >= (1u << 20)) {  // the repair after the batch settles x
+            if (lane_id() == 0) atomicOr(g.err, ERR_RETRY);
+            return;
+        }
+        cur = got;
+        newc = warp_fac(g, x, g.st);
+        if (newc == color_of(cur)) return;
+    }
+    if (lane_id() == 0) {
+        mark_touched(g, x);
+        note_color(g, x);
+    }
+    const uint16_t oldc = color_of(cur);
+    const uint64_t s = g.rp[x], e = live_end(g, x, s);
+    warp_for_each(g.col, s, e, [&](uint64_t, uint32_t ng) {
+        if (ng == INV || ng >= g.n) return;
+        nbr_color_change(g, ng, oldc, newc);
+    });
+    __syncwarp();
+}
+__device__ __forceinline__ void warp_recolor(const Dev& g, uint32_t x, uint16_t chosen = 0) {
+    warp_recolor_from(g, x, chosen, warp_load_state(g, x));
+}
+
+// Warp-collective: does some live neighbor of x hold color c? Stops at the
+// first round that finds one.
+__device__ __forceinline__ bool warp_color_held(const Dev& g, uint32_t x, uint16_t c) {
+    const uint64_t s = g.rp[x], e = live_end(g, x, s);
+    // rounds of 128 slots: a holder is usually among the first neighbors
+    return warp_gather_each<true, 1>(g.col, s, e, g.n, g.st, [c](uint32_t, uint32_t w) { return color_of(w) == c; });
+}
+
+// Does a live neighbor among the first `lim` live slots of x hold color c?
+// `all`: those slots were the whole row.
+__device__ __forceinline__ bool warp_color_held_first(const Dev& g, uint32_t x, uint16_t c, uint32_t lim, bool& all) {
+    const uint64_t s = g.rp[x], e = live_end(g, x, s);
+    const uint64_t e1 = e - s > lim ? s + lim : e;
+    all = e1 == e;
+    return warp_gather_each<true, 4>(g.col, s, e1, g.n, g.st, [c](uint32_t, uint32_t w) { return color_of(w) == c; });
 }
 
 // Appends a row-scale operation to the pass after the batch (lane 0).
@@ -752,140 +818,142 @@ __device__ __forceinline__ bool warp_defer(const Dev& g, uint32_t x, uint32_t ki
     return __shfl_sync(FULL, ok, 0) != 0;
 }
 
-// ---------------- one update of a concurrent batch (local_update.cu:61-147) ----------------
-//
-// What an update can end with, at most once per endpoint: coloring an uncolored
-// endpoint, recoloring the loser of a conflict (recolor_vertex), or moving to a
-// lower color after a delete freed one (try_color_reduction). One loop holds the
-// only copy of the selection and the walk: with them inlined at each place the
-// kernel's warps, each somewhere else in it, waited for instructions 40 % of the
-// time.
-enum : uint32_t { ACT_COLOR, ACT_RECOLOR, ACT_REDUCE };
-
-// One such act on x (warp-collective); `state` is x's state word as the caller
-// last read it. Returns x's state word afterwards.
-__device__ __forceinline__ uint32_t warp_act(const Dev& g, uint32_t x, uint32_t act, uint16_t freed, uint32_t state) {
-    uint32_t newc = 0, cur = act == ACT_RECOLOR ? ld_cg(g.st + x) : state;
-    if (act == ACT_REDUCE) {
-        if (color_of(state) == 0 || freed >= color_of(state)) return state;
-        if (g.exact && __ldg(g.hdmap + x) != EMPTY) {
-            // A row above the threshold moves to `freed` when no live neighbor
-            // holds it any more (an early-exit scan; the full scan of a
-            // high-degree row would almost always confirm the current color). A
-            // holder is usually among the first neighbors; a hub row without one
-            // there is finished (scan, move, walk) by the pass after the batch.
-            if (freed == 0) return state;
-            const uint64_t s = g.rp[x], e = live_end(g, x, s);
-            uint64_t from = s, to = g.hub_ops && e - s > kHubRow ? s + kHubScan : e;
-            for (;;) {
-                if (warp_color_held(g, from, to, freed)) return state;
-                if (to == e) break;
-                if (warp_defer(g, x, HUB_REDUCE, freed)) return state;
-                from = s;
-                to = e;
-            }
-            newc = freed;
-        }
-    }
-    uint16_t oldc;
-    for (uint32_t tries = 0;; tries++) {
-        if (newc == 0) newc = warp_fac(g, x, g.st);
-        if (act == ACT_REDUCE && tries == 0) {
-            if (newc >= color_of(state)) return state;
-            cur = ld_cg(g.st + x);
-        }
-        oldc = color_of(cur);
-        if (act != ACT_COLOR && newc == oldc) return cur;
-        const uint32_t want = pack((uint16_t)newc, act == ACT_COLOR ? (uint16_t)1 : (uint16_t)(version_of(cur) + 1));
-        uint32_t got = 0;
-        if (lane_id() == 0) got = atomicCAS(g.st + x, cur, want);
-        got = __shfl_sync(FULL, got, 0);
-        if (got == cur) {
-            cur = want;
-            break;
-        }
-        if (act == ACT_COLOR) return got;  // another warp's color came first
-        if (tries >= (1u << 20)) {         // the repair after the batch settles x
-            if (lane_id() == 0) atomicOr(g.err, ERR_RETRY);
-            return got;
-        }
-        cur = got;
-        newc = 0;
-    }
-    if (lane_id() == 0) {
-        mark_touched(g, x);
-        note_color(g, x);
-    }
-    if (act != ACT_COLOR) {
-        const uint64_t s = g.rp[x];
-        warp_walk(g, s, live_end(g, x, s), oldc, (uint16_t)newc);
-    }
-    return cur;
+// Both endpoints' state words in one round trip (lanes 0 and 1).
+__device__ __forceinline__ void warp_load_states2(const Dev& g, uint32_t u, uint32_t v, uint32_t& su, uint32_t& sv) {
+    const uint32_t lane = lane_id();
+    uint32_t w = 0;
+    if (lane < 2) w = ld_cg(g.st + (lane ? v : u));
+    su = __shfl_sync(FULL, w, 0);
+    sv = __shfl_sync(FULL, w, 1);
 }
 
-__device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v, uint8_t type) {
-    if (type != SGC_UPDATE_ADD && type != SGC_UPDATE_DEL) return;
-    const bool add = type == SGC_UPDATE_ADD;
-    // The two row edits of an edge (u != v) touch two different rows and no
-    // other warp edits those slots of theirs, so the two halves of the warp make
-    // them at once (lanes 0-15 row u, 16-31 row v).
-    const Lanes<16> H;
-    const uint32_t x = H.base ? v : u, y = H.base ? u : v;
-    const uint32_t hd = __ldg(g.hdmap + x);
-    uint32_t st = add ? 0u : ld_cg(g.st + x);  // a delete: as they were before it
-    int r = 0;
-    for (uint32_t turn = 0; turn < (u == v ? 2u : 1u); turn++) {  // a self loop: one half after the other
-        if (u != v || (H.base != 0) == (turn != 0)) r = grp_edit_row(H, g, x, y, add);
-        __syncwarp();
+// try_color_reduction in a concurrent batch: after a delete freed `freed`, move
+// to a lower color if one is open. With exact selection on a row above the
+// threshold, instead of the full first-free scan, x moves to `freed` when no
+// live neighbor holds it any more (an early-exit scan; the full scan of a
+// high-degree row would almost always confirm the current color). `state` is
+// x's state word as the caller last read it (a recolor re-reads it).
+__device__ __forceinline__ void warp_try_reduce(const Dev& g, uint32_t x, uint16_t freed, uint32_t state) {
+    const uint16_t cur = color_of(state);
+    if (cur == 0) return;
+    if (freed >= cur) return;
+    if (g.exact && __ldg(g.hdmap + x) != EMPTY) {
+        if (freed == 0) return;
+        if (g.hub_ops && row_len(g, x) > kHubRow) {
+            // a holder is usually among the first neighbors; a hub row without
+            // one there is finished (scan, move, walk) by the pass after the batch
+            bool all = true;
+            if (warp_color_held_first(g, x, freed, kHubScan, all)) return;
+            if (warp_defer(g, x, HUB_REDUCE, freed) || warp_color_held(g, x, freed)) return;
+        } else if (warp_color_held(g, x, freed)) {
+            return;
+        }
+        warp_recolor(g, x, freed);
+        return;
     }
-    if (__shfl_sync(FULL, r, 0) != __shfl_sync(FULL, r, 16) && lane_id() == 0) flag_asym(g, u);
-    // Bitmap-class rows are revisited by the next repair (their bitmaps rebuilt);
-    // a row with a histogram class takes exact colors from its live neighbors
-    // instead, and is revisited only when its color changes or an ADD leaves a
-    // conflict.
-    if (hd == EMPTY && H.leader()) mark_touched(g, x);
-    // An insert reads the state words once, after the row edits, and keeps them:
-    // a later change by another warp is a color change (marked) or leaves this
-    // ADD's endpoints equal (caught by the check after the batch).
-    if (add) st = ld_cg(g.st + x);
-    uint32_t su = __shfl_sync(FULL, st, 0), sv = __shfl_sync(FULL, st, 16);
-    uint16_t fu = 0, fv = 0;
-    // 0, 1: color u, then v (inserts that meet an uncolored endpoint); 2: the
-    // loser of a conflict, or reduce u; 3: reduce v
-    for (uint32_t k = add && (color_of(su) == 0 || color_of(sv) == 0) ? 0u : 2u; k < (add ? 3u : 4u); k++) {
-        uint32_t z = k & 1u ? v : u, act = k < 2 ? ACT_COLOR : ACT_REDUCE;
-        if (k < 2) {
-            if (color_of(k ? sv : su) != 0) continue;
-            if (k && lane_id() == 0) new_nbr(g, v, color_of(su));
-        } else if (k == 2) {
-            const uint16_t oc = color_of(H.base ? su : sv);  // the other endpoint's
-            if (H.leader() && oc != 0) {
-                if (add && oc <= 64) set_bm_bit<false>(g, x, oc);
-                if (hd != EMPTY && !g.exact && oc <= g.maxc)  // new_nbr, removed_nbr
-                    atomicAdd(g.hist + (uint64_t)hd * g.maxc + oc - 1, add ? 1u : ~0u);
-            }
-            fu = color_of(sv);
-            fv = color_of(su);
-            if (add) {
-                if (fu != fv || fu == 0) break;
-                z = prio_less(__ldg(g.deg + u), u, __ldg(g.deg + v), v) ? u : v;
-                // a long histogram-class row's selection and walk go to the pass after the batch
-                if (g.hub_ops && __ldg(g.hdmap + z) != EMPTY && row_len(g, z) > kHubRow &&
-                    warp_defer(g, z, HUB_RECOLOR, 0))
-                    break;
-                act = ACT_RECOLOR;
-            }
-        } else if (u == v) {
-            sv = ld_cg(g.st + v);
+    const uint16_t best = warp_fac(g, x, g.st);
+    if (best < cur) warp_recolor(g, x, best);
+}
+
+// Colors x, read uncolored as state word `cur`, with FAC; version becomes 1
+// (local_update.cu:90-101). Returns x's state word afterwards (another warp's
+// color if it got there first).
+__device__ __forceinline__ uint32_t warp_color_uncolored(const Dev& g, uint32_t x, uint32_t cur) {
+    const uint16_t c = warp_fac(g, x, g.st);
+    uint32_t got = 0;
+    if (lane_id() == 0) {
+        const uint32_t want = pack(c, 1);
+        const uint32_t old = atomicCAS(g.st + x, cur, want);
+        if (old == cur) {
+            mark_touched(g, x);
+            note_color(g, x);
+            got = want;
+        } else {
+            got = old;
+        }
+    }
+    return __shfl_sync(FULL, got, 0);
+}
+
+// ---------------- one update of a concurrent batch (local_update.cu:61-147) ----------------
+
+__device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v, uint8_t type) {
+    if (g.touched && lane_id() == 0 && (type == SGC_UPDATE_ADD || type == SGC_UPDATE_DEL)) {
+        // bitmap-class rows are revisited (their bitmaps rebuilt); a row with a
+        // histogram class takes exact colors from its live neighbors instead,
+        // and is revisited only when its color changes or an ADD leaves a conflict
+        if (__ldg(g.hdmap + u) == EMPTY) mark_touched(g, u);
+        if (__ldg(g.hdmap + v) == EMPTY) mark_touched(g, v);
+    }
+    // The state words are read once, after the row edits, and kept: a later
+    // change by another warp is a color change (marked) or leaves this ADD's
+    // endpoints equal (caught by the check after the batch).
+    // The two row edits of an edge (u != v) touch two different rows and no
+    // other warp edits those slots of theirs, so the two halves of the warp
+    // make them at once (lanes 0-15 row u, 16-31 row v).
+    const bool halves = u != v;
+    if (type == SGC_UPDATE_ADD) {
+        int ru, rv;
+        if (halves) {
+            const Lanes<16> H;
+            const uint32_t x = H.base ? v : u, y = H.base ? u : v;  // one call site: the halves stay converged
+            const int r = grp_add_slot(H, g, x, y);
+            __syncwarp();
+            ru = __shfl_sync(FULL, r, 0);
+            rv = __shfl_sync(FULL, r, 16);
+        } else {
+            ru = warp_add_slot(g, u, v);
+            rv = warp_add_slot(g, v, u);
+        }
+        if (ru != rv && lane_id() == 0) flag_asym(g, u);
+        uint32_t su, sv;
+        warp_load_states2(g, u, v, su, sv);
+        if (color_of(su) == 0) {
+            su = warp_color_uncolored(g, u, su);
+            if (v == u) sv = su;
+        }
+        if (color_of(sv) == 0) {
+            if (lane_id() == 0) new_nbr(g, v, color_of(su));
+            __syncwarp();
+            sv = warp_color_uncolored(g, v, sv);
+        }
+        if (lane_id() == 0) new_nbr(g, u, color_of(sv));
+        else if (lane_id() == 1) new_nbr(g, v, color_of(su));
+        __syncwarp();
+        const uint16_t cu = color_of(su), cv = color_of(sv);
+        if (cu == cv && cu != 0) {
+            const uint32_t loser = prio_less(__ldg(g.deg + u), u, __ldg(g.deg + v), v) ? u : v;
+            // a long histogram-class row's selection and walk go to the pass after the batch
+            const bool defer = g.hub_ops && __ldg(g.hdmap + loser) != EMPTY && row_len(g, loser) > kHubRow &&
+                               warp_defer(g, loser, HUB_RECOLOR, 0);
+            if (!defer) warp_recolor(g, loser);
+        }
+    } else if (type == SGC_UPDATE_DEL) {
+        uint32_t su, sv;
+        warp_load_states2(g, u, v, su, sv);
+        const uint16_t fu = color_of(sv);
+        const uint16_t fv = color_of(su);
+        bool du, dv;
+        if (halves) {
+            const Lanes<16> H;
+            const uint32_t x = H.base ? v : u, y = H.base ? u : v;
+            const int d = grp_remove_slot(H, g, x, y) ? 1 : 0;
+            __syncwarp();
+            du = __shfl_sync(FULL, d, 0) != 0;
+            dv = __shfl_sync(FULL, d, 16) != 0;
+        } else {
+            du = warp_remove_slot(g, u, v);
+            dv = warp_remove_slot(g, v, u);
+        }
+        if (lane_id() == 0) {
+            if (du != dv) flag_asym(g, u);
+            removed_nbr(g, u, fu);
+            removed_nbr(g, v, fv);
         }
         __syncwarp();
-        const uint32_t w = warp_act(g, z, act, k & 1u ? fv : fu, k & 1u ? sv : su);
-        if (k == 0) {
-            su = w;
-            if (u == v) sv = w;
-        } else if (k == 1) {
-            sv = w;
-        }
+        warp_try_reduce(g, u, fu, su);
+        if (v == u) sv = warp_load_state(g, v);
+        warp_try_reduce(g, v, fv, sv);
     }
 }
 

@@ -650,7 +650,7 @@ __device__ __forceinline__ bool warp_drain_insert(const Dev& g, uint32_t x, uint
     uint64_t from = s;
     if (!ordered && g.blen) {
         const uint32_t bl = ld_cg(g.blen + x);
-        if (bl && warp_run_add(g, x, nbr, s, bl)) return true;
+        if (bl && warp_run_add(g, x, nbr, s, bl) >= 0) return true;
         from = s + bl;
     }
     for (;;) {
