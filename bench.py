@@ -269,7 +269,7 @@ def run_ours(a):
     t = time.time()
     # no periodic full repair: every published snapshot is checked by the validator instead.
     # Profiling times the sweeps of eager repairs (the full repair after the run); a
-    # captured publish runs its sweeps inside one graph launch.
+    # default publish runs its sweeps inside one kernel.
     h = S.StreamGC(g, epoch_size=E, histogram_threshold=HIST_THR, slack_pct=300, max_batch=1 << 20,
                    device=local, profile=True, exact_select=True, graph_publish=a.graph_publish,
                    sorted_rows=a.sorted_rows, full_repair_every=a.full_repair_every)
@@ -408,7 +408,7 @@ def run_ours(a):
         roof_sweep = {"bound": "hbm", "kernel": "tier-1 sweep (sweep_items + finalize + fac + commit)",
                       "achieved": achieved, "peak": peak, "unit": "GB/s",
                       "frac": achieved / peak if achieved is not None else None, "peak_kind": pk,
-                      "note": None if achieved is not None else "sweeps run inside the captured publish graph "
+                      "note": None if achieved is not None else "sweeps run inside the publish's one kernel "
                               "and are not timed one by one; roofline_full_sweep times them over every vertex",
                       "traffic": traffic, "algorithmic_bytes_per_sweep": sweep_bytes / max(1, sweeps),
                       "sweep_ms_avg": sweep_ms / max(1, sweeps), "sweeps_timed": sweeps}
@@ -425,7 +425,7 @@ def run_ours(a):
                           "algorithmic_bytes_per_launch": bpu * E, "apply_ms_avg": apply_avg}
         conf = dict(desc)
         conf.update(mode="concurrent (warp per edge) + repaired publish per epoch, exact color selection"
-                    + (", publish as one CUDA graph" if a.graph_publish else "")
+                    + (", repair loop as one kernel" if a.graph_publish else "")
                     + (", e2e through the ingest slots" if a.ingest else "")
                     + (", rows kept as one sorted run" if a.sorted_rows else ""),
                     l2="flushed before every timed step (256 MiB write)", parallelism=f"replicas x{world}",
@@ -1040,7 +1040,7 @@ def main():
                          "batch overlapping this epoch's publish)")
     ap.add_argument("--eager-publish", dest="graph_publish", action="store_false",
                     help="plain path: publish with one host round trip per repair sweep instead of replaying "
-                         "the captured publish graph (SGC_OPT_GRAPH_PUBLISH, the default)")
+                         "the one kernel of the whole loop (SGC_OPT_GRAPH_PUBLISH, the default)")
     ap.add_argument("--graph-publish", dest="graph_publish", action="store_true", help=argparse.SUPPRESS)
     ap.add_argument("--epoch-size", type=int, default=32768,
                     help="plain path: updates per epoch (the large workload's sweep uses 4096, 32768, 262144)")
