@@ -165,7 +165,7 @@ __global__ void conc_prep_insert(Dev g, const EdgeUpdate* __restrict__ ups, uint
         // Double hashing (an odd step visits every slot of the power-of-two table):
         // the kernel's time is its longest chain of probes, which at half load is
         // near log2(n) this way but over fifty slots' cluster in a row with step 1
-        // (65,536 updates: 16 us, now 9).
+        // (an epoch of 65,536 updates, this kernel 16 us of it, became 7 us shorter).
         const unsigned long long mix = key_hash(key);
         const uint32_t step = (uint32_t)(mix >> 32) | 1u;
         uint32_t h = (uint32_t)mix & eo.tmask;
@@ -515,8 +515,8 @@ constexpr uint32_t kMergeMax = 1024;
 
 // Ascending bitonic sort of buf[0, m), m a power of two: only as many slots as
 // the row fills. (Sorting kMergeMax slots for every row made 55 rounds over 32
-// slots per lane of a row of twenty entries: the compaction of 30,000 rows took
-// 114 us, against 36 with rows sorted at their own size.)
+// slots per lane of a row of twenty entries, most of the 114 us that an epoch's
+// compaction took on a Chung-Lu graph of 300,007 vertices.)
 __device__ __forceinline__ void warp_sort_row(uint32_t* buf, uint32_t m, uint32_t lane) {
     for (uint32_t k = 2; k <= m; k <<= 1)
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
@@ -538,7 +538,7 @@ __device__ __forceinline__ void warp_sort_row(uint32_t* buf, uint32_t m, uint32_
 // round; the warp then compacts, one after another, those that need it. (A warp
 // per row spent two round trips on each row it left alone: 16 us for the 50,000
 // rows of an epoch of 32,768 updates on a mesh, 67 us for 262,144 on a power-law
-// graph; now 8 and 30.) One thread takes the overflow count for the drain that
+// graph. With it the epochs became 8 and 60 us shorter.) One thread takes the overflow count for the drain that
 // follows (`drain_n` non-null); nothing appends to the buffer meanwhile.
 __global__ void __launch_bounds__(256) compact_kernel(Dev g, const uint32_t* __restrict__ list,
                                                       const uint32_t* __restrict__ count, int force, int merge,
@@ -763,7 +763,7 @@ constexpr uint32_t kTailBlocks = 16, kTailList = 2048, kTailItems = 768;
 // of the list sit on different SMs. A list shorter than the grid then occupies
 // every SM a little instead of the first few fully: loading a Chung-Lu graph of
 // 300,007 vertices took 4.73 ms with consecutive warps in one block and 4.14 this
-// way, epochs on a mesh of 131,072 vertices 189 and 184 us. (The reference
+// way, epochs on a mesh of 131,072 vertices became 5 us shorter. (The reference
 // rules' first sweep, which visits every vertex in order, lost 1 % with it.)
 __device__ __forceinline__ uint32_t spread_warp(uint32_t nb) { return (threadIdx.x >> 5) * nb + blockIdx.x; }
 
@@ -1641,11 +1641,11 @@ __device__ __forceinline__ void sweep_long(const Dev& g, const SweepBufs& b, int
 // A vertex takes the first color in 1..2047 that no neighbor in its row holds
 // (2048 when all are held), version 1; colors given earlier in the list count,
 // vertices already colored are passed over. One vertex after another, a block on
-// each row, took 1.5 to 3.3 us per vertex: a dependent chain of its loads. So the
+// each row, was a dependent chain of loads per vertex: 2.2 ms for the core of a
+// Chung-Lu graph of 300,007 vertices, 0.77 ms this way. The
 // list is taken a window at a time: a block per vertex gathers the colors its
 // neighbors hold and which earlier vertices of the window are among them, and
 // then one warp colors the window in order from those sets in shared memory.
-// 80 ns per vertex there, and the gathers of a window overlap: 0.15 us per vertex.
 
 // place[v]: 1 + v's place in the list (0: not in it).
 __global__ void list_places_kernel(const uint32_t* __restrict__ list, uint32_t m, uint32_t* place) {

@@ -375,8 +375,8 @@ __global__ void row_total_kernel(Dev g, unsigned long long* total) {
 
 // Every slot's edge as a key (lower endpoint << bits | higher), bit 2 * bits set
 // where the slot holds none. A warp takes 32 rows and their room in `keys` with
-// one atomic (one per entry, on one word, was 1.0 ms of a graph with 8 M entries;
-// now 0.1), then writes row by row.
+// one atomic (one per entry, on one word, took 1.0 ms for 8 M entries), then
+// writes row by row.
 __global__ void __launch_bounds__(256) validate_kernel(Dev g, unsigned long long* keys, uint32_t bits,
                                                        unsigned long long* words /* uncolored, max color, oor, -, -, cursor */) {
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5, lane = lane_id();
