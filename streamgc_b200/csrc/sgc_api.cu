@@ -548,6 +548,7 @@ int sgci::create_internal(const StreamGCConfig* cfg, const sgc_options* opt_in, 
     A(&sb.wl, n);
     A(&sb.wl_count, 4, 0);
     sb.next_items = sb.wl_count + 1;
+    sb.seed_count = sb.wl_count + 2;
     A(&sb.swept, 2, 0);
     A(&sb.needf, n, 0);
     A(&sb.need_v, n);

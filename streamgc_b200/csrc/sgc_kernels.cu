@@ -1401,8 +1401,8 @@ __global__ void repair_begin_kernel(Dev g, SweepBufs b) { repair_begin(g, b); }
 
 // First worklist of an independent-set repair: every vertex of the graphs
 // repaired in full, the touched vertices of the others; clears the touched
-// marks. Thread per 32-vertex word.
-__device__ __forceinline__ void seed_worklist(const Dev& g, const SweepBufs& b, uint32_t nb) {
+// marks; the list's length goes to *count. Thread per 32-vertex word.
+__device__ __forceinline__ void seed_worklist(const Dev& g, const SweepBufs& b, uint32_t nb, uint32_t* count) {
     const uint32_t nw = (g.n + 31) / 32;
     for (uint32_t base = spread_warp(nb) * 32; base < nw; base += nb * blockDim.x) {
         const uint32_t w = base + lane_id();
@@ -1417,10 +1417,10 @@ __device__ __forceinline__ void seed_worklist(const Dev& g, const SweepBufs& b, 
                 bits = t;
             }
         }
-        list_bits(w, bits, b.wl, b.wl_count);
+        list_bits(w, bits, b.wl, count);
     }
 }
-__global__ void seed_worklist_kernel(Dev g, SweepBufs b) { seed_worklist(g, b, gridDim.x); }
+__global__ void seed_worklist_kernel(Dev g, SweepBufs b) { seed_worklist(g, b, gridDim.x, b.wl_count); }
 
 // After each sweep: reads the counts, decides whether another sweep runs,
 // advances the index. Reference rule (TIER1): stop at 0 conflicts, after 3
@@ -1771,9 +1771,28 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
             *b.need_count = 0;
         }
     };
+    // Block 0 between two sweeps: what the next one visits and who runs it. The
+    // count of the list it visits is kept in the control block and its words are
+    // made zero here, where no other block runs: the collection at the sweep's end
+    // adds to them, and a sweep that finds no conflict has no barrier before it.
+    auto plan = [&](bool counted) {
+        if (threadIdx.x != 0) return;
+        const uint32_t lim = rc.list ? *b.wl_count : g.n;
+        const uint32_t next = counted ? *b.next_items : NONE32;
+        uint32_t go = SWEEP_ELSEWHERE;
+        if (rc.cont && lim <= most) {
+            if (sync.nb > kTailBlocks) go = lim <= kTailList && next <= kTailItems ? SWEEP_TAIL : SWEEP_GRID;
+            else if (lim <= 4 * kTailList && next <= 4 * kTailItems) go = SWEEP_TAIL;  // else another launch goes on
+        }
+        rc.go = go;
+        rc.lim = lim;
+        if (go == SWEEP_ELSEWHERE) return;  // the kernels that go on read the list's length there
+        *b.wl_count = 0;
+        *b.next_items = 0;
+    };
     if (!sync.serial([&] {
             reset();
-            if (threadIdx.x == 0) *b.next_items = NONE32;  // not counted for the first list
+            if (threadIdx.x == 0) *b.seed_count = 0;
             if (start) {
                 if (threadIdx.x == 0) {
                     rc.mode = in.mode;
@@ -1782,38 +1801,35 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
                 }
                 __syncthreads();
                 repair_begin(g, b);
+                __syncthreads();
             }
+            plan(false);
         }))
         return false;
     const int mode = (int)rc.mode;
     const bool indep = mode == SWEEP_INDEP;
-    if (start && indep) {
-        seed_worklist(g, b, sync.nb);
+    uint32_t go = rc.go, lim = rc.lim;
+    if (start && indep) {  // the first list, which has a counter of its own
+        seed_worklist(g, b, sync.nb, b.seed_count);
         if (!sync()) return false;
+        lim = *b.seed_count;
+        go = lim <= most ? SWEEP_GRID : SWEEP_ELSEWHERE;
+        if (go == SWEEP_ELSEWHERE && tid == 0) *b.wl_count = lim;
     }
     bool recolored = false;  // bits set in b.rbits
     for (;;) {
         if (recolored)
             for (uint32_t w = tid; w < nw; w += sync.nb * blockDim.x) b.rbits[w] = 0;
+        if (go == SWEEP_ELSEWHERE) return true;
         const bool list = rc.list != 0;
-        const uint32_t lim = list ? *b.wl_count : g.n;
-        if (!rc.cont || lim > most) return true;
-        if (sync.nb > kTailBlocks) {
-            if (lim <= kTailList && *b.next_items <= kTailItems) {
-                sync.nb = kTailBlocks;
-                if (blockIdx.x >= kTailBlocks) return true;
-            }
-        } else if (lim > 4 * kTailList || *b.next_items > 4 * kTailItems) {
-            return true;  // grown again: another launch goes on
+        if (go == SWEEP_TAIL && sync.nb > kTailBlocks) {
+            sync.nb = kTailBlocks;
+            if (blockIdx.x >= kTailBlocks) return true;
         }
         const uint32_t nb = sync.nb;
         const bool sym = want_sym(b, 2);
         sweep_short(g, b, mode, list, lim, sym, nb);
         if (!sync()) return false;
-        if (tid == 0) {  // every block has read them
-            *b.wl_count = 0;
-            *b.next_items = 0;
-        }
         const uint32_t items = *b.item_count < b.item_cap ? *b.item_count : b.item_cap;
         if (items) {
             sweep_items(g, b, mode, 2, nb);
@@ -1847,8 +1863,11 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
                 repair_step(g, b);
                 __syncthreads();
                 reset();
+                plan(true);
             }))
             return false;
+        go = rc.go;
+        lim = rc.lim;
     }
 }
 __global__ void __launch_bounds__(kFusedThreads, 1) repair_fused_kernel(Dev g, SweepBufs b, int start, RepairIn in,

@@ -29,7 +29,9 @@ struct RepairCtl {
     uint32_t next;         // size of the next worklist
     uint32_t prev;         // reference rule: last count
     uint32_t plateau;      // reference rule: equal counts in a row
-    uint32_t pad[3];
+    uint32_t go;           // one-kernel repair: SWEEP_* of the next sweep
+    uint32_t lim;          // one-kernel repair: vertices it visits
+    uint32_t pad;
     unsigned long long sym;   // nonzero: some graph's first-sweep checksum was not 0
     unsigned long long live;  // first sweep's live entries
     unsigned long long swept[2];  // live entries and vertices visited by the sweeps so far
@@ -38,6 +40,10 @@ struct RepairCtl {
 struct RepairIn {
     uint32_t mode, max_sweeps, force_all;
 };
+
+// Who runs the next sweep of a one-kernel repair: other kernels (or none does),
+// the whole grid, or its first few blocks.
+enum : uint32_t { SWEEP_ELSEWHERE = 0, SWEEP_GRID = 1, SWEEP_TAIL = 2 };
 
 // Barrier across the blocks of a cooperative launch (one per handle).
 struct GridBar {
@@ -70,6 +76,7 @@ struct SweepBufs {
     uint32_t* wl;
     uint32_t* wl_count;
     uint32_t* next_items;        // work items the next worklist will make
+    uint32_t* seed_count;        // one-kernel repair: length of its first worklist
     unsigned long long* swept;   // [0] live entries, [1] vertices visited by the sweeps since reset
     // independent-set sweeps: conflicted vertices of the current sweep
     uint8_t* needf;              // per vertex: conflicted (or uncolored with neighbors) at the last visit
