@@ -1568,6 +1568,17 @@ struct GridSync {
         }
         return __syncthreads_and(ok);
     }
+    // The grid goes on with its first `k` blocks: the others call part() and return.
+    // Their last arrivals are awaited at the next barrier of those that stay, so
+    // what they still read or write comes before anything after that barrier.
+    __device__ __forceinline__ void part() {
+        __syncthreads();
+        if (threadIdx.x == 0) arrive();
+    }
+    __device__ __forceinline__ void shrink(uint32_t k) {
+        due += nb - k;
+        nb = k;
+    }
     // The same, where block 0 runs `last` when all have arrived, before any goes on.
     template <class F>
     __device__ __forceinline__ bool serial(F last) {
@@ -1823,8 +1834,11 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
         if (go == SWEEP_ELSEWHERE) return true;
         const bool list = rc.list != 0;
         if (go == SWEEP_TAIL && sync.nb > kTailBlocks) {
-            sync.nb = kTailBlocks;
-            if (blockIdx.x >= kTailBlocks) return true;
+            if (blockIdx.x >= kTailBlocks) {  // the decision is read, its share of the recolored bits cleared
+                sync.part();
+                return true;
+            }
+            sync.shrink(kTailBlocks);
         }
         const uint32_t nb = sync.nb;
         const bool sym = want_sym(b, 2);
