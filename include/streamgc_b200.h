@@ -28,7 +28,8 @@ typedef struct sgc_handle sgc_handle;
 #define SGC_EINVAL      -1   /* bad argument */
 #define SGC_ECUDA       -2   /* CUDA runtime error */
 #define SGC_ENOMEM      -3   /* device or host allocation failed */
-#define SGC_EDEVICE     -4   /* device-side error word set (see sgc_stats.device_error) */
+#define SGC_EDEVICE     -4   /* device-side error word set (see sgc_stats.device_error), or a repair or core
+                                coloring gave up at a barrier: no snapshot was published, the next repair is full */
 #define SGC_ENOTSUP     -5   /* request outside this library's single-GPU scope */
 
 /* update-application modes */
@@ -105,7 +106,8 @@ typedef struct sgc_stats {
     uint64_t tier1_sweeps;       /* cumulative */
     uint64_t tier2_runs;
     uint64_t tier2_fixed;
-    uint32_t device_error;       /* bit 0: wait timeout, bit 1: bad update, bit 2: list overflow */
+    uint32_t device_error;       /* bit 0: wait timeout, bit 1: bad update, bit 2: list overflow, bit 3: order of
+                                    same-edge updates, bit 4: color retries, bit 5: row mark, bit 6: barrier */
     uint32_t num_vertices;
     uint32_t num_high_degree;
     uint32_t max_hist_colors;    /* histogram bins per row kept on the device (0 with SGC_OPT_EXACT_SELECT) */

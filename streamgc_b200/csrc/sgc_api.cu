@@ -205,14 +205,21 @@ int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool tim
         if (!rc->cont) break;
     }
     TRY(check_cuda("repair"));
+    TRY(finish_repair(h, rep));
     if (h->opt.flags & (SGC_OPT_PROFILE | SGC_OPT_GRAPH_PUBLISH)) h->sweep_bytes += 8ull * rc->swept[0] + 28ull * rc->swept[1];
-    return finish_repair(h, rep);
+    return SGC_OK;
+}
+
+// SGC_EDEVICE for a control block that a one-kernel repair gave up on.
+int check_repair(const RepairCtl& rc) {
+    return rc.fault ? fail(SGC_EDEVICE, "repair: a barrier across the grid gave up") : SGC_OK;
 }
 
 // After the Tier-1 loop (its control block read back into h_rc_out): the
 // counters, and Tier-2 when the loop did not leave a proper coloring.
 int finish_repair(sgc_handle* h, sgc_repair_report* rep) {
     const RepairCtl* rc = h->h_rc_out;
+    TRY(check_repair(*rc));
     h->tier1_sweeps += rc->it;
     if (!rc->incr) h->live_entries = rc->live;
     h->repairs_since_full = rc->incr ? h->repairs_since_full + 1 : 0;
@@ -1022,6 +1029,7 @@ int sgc_color_core(sgc_handle* h, uint32_t min_degree, uint32_t* colored) {
         TRY(sync(h));
         TRY(check_cuda("color_core"));
         done = h->h_small[0];
+        if (done == NONE32) return fail(SGC_EDEVICE, "color_core: a barrier across the grid gave up");
     }
     if (colored) *colored = done;
     return SGC_OK;

@@ -499,6 +499,12 @@ int sgc_batch_tick_end(sgc_batch* b, sgc_batch_tick_report* rep) {
     TRY(check_cuda("batch tick"));
     const RepairCtl rc = *h->h_rc_out;
     h->d2h_bytes += sizeof(RepairCtl);
+    if (const int r = check_repair(rc)) {  // the updates are applied; no snapshot changes, the epochs close at the next tick
+        h->updates += nup;
+        for (uint32_t k = 0; k < G; k++)
+            if (b->h_target[k] < 2) b->close_one[k] = 1;
+        return r;
+    }
     bool proper = rc.done && rc.sym == 0;
     uint32_t t2 = 0;
     if (!proper) {  // sequential fallback, then publish again

@@ -1384,6 +1384,7 @@ __device__ __forceinline__ void repair_begin(const Dev& g, const SweepBufs& b) {
         rc.it = 0;
         rc.cont = 1;
         rc.done = 0;
+        rc.fault = 0;
         rc.need = 0;
         rc.next = 0;
         rc.prev = 0xFFFFFFFFu;
@@ -1599,14 +1600,22 @@ struct GridSync {
         }
         return true;
     }
-    // The last block to leave makes the words zero for the next launch.
-    __device__ __forceinline__ void leave() {
+    // Every block ends here, `ok` false where a barrier gave up on it. The last one
+    // makes the words zero for the next launch and, on its thread 0 alone, returns
+    // true; `ok` then says whether all blocks met at every barrier.
+    __device__ __forceinline__ bool leave(bool& ok) {
         __syncthreads();
-        if (threadIdx.x == 0 && atomicAdd(&bar->left, 1u) == gridDim.x - 1) {
-            bar->count = 0;
-            bar->gen = 0;
-            bar->left = 0;
-        }
+        if (threadIdx.x != 0) return false;
+        fence_gpu();
+        const uint32_t before = atomicAdd(&bar->left, ok ? 1u : 0x10001u);  // blocks, and those given up on above
+        if ((before & 0xFFFFu) != gridDim.x - 1) return false;
+        fence_gpu();
+        ok = ok && before < 0x10000u;
+        bar->count = 0;
+        bar->gen = 0;
+        bar->left = 0;
+        bar->failed = 0;
+        return true;
     }
 };
 
@@ -1742,7 +1751,7 @@ __global__ void __launch_bounds__(kColorThreads, 1) color_list_kernel(Dev g, con
         ok = sync();
     }
     if (blockIdx.x == 0 && tid == 0) *colored = done;
-    sync.leave();
+    if (sync.leave(ok) && !ok) *colored = NONE32;
 }
 void launch_color_list(const Dev& g, const uint32_t* list, uint32_t m, uint32_t* place, uint32_t* rows, GridBar* bar,
                        uint32_t* colored, int num_sms, cudaStream_t s) {
@@ -1889,9 +1898,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) repair_fused_kernel(Dev g, S
                                                                         cudaGraphConditionalHandle cond,
                                                                         int has_cond) {
     GridSync sync(b.bar, g.err);
-    const bool ok = repair_fused(g, b, sync, start, in, most);
-    sync.leave();
-    if (has_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, ok ? b.rc->cont : 0u);
+    bool ok = repair_fused(g, b, sync, start, in, most);
+    if (!sync.leave(ok)) return;
+    RepairCtl& rc = *b.rc;
+    if (!ok) {  // nothing in the block may be taken for a result; the next repair visits every vertex
+        rc.fault = 1;
+        rc.cont = 0;
+        for (uint32_t k = 0; k < b.G; k++) g.gctl[k].clean = 0;
+    }
+    if (has_cond) cudaGraphSetConditional(cond, rc.cont);
 }
 
 void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start, int num_sms, cudaStream_t s,

@@ -31,7 +31,7 @@ struct RepairCtl {
     uint32_t plateau;      // reference rule: equal counts in a row
     uint32_t go;           // one-kernel repair: SWEEP_* of the next sweep
     uint32_t lim;          // one-kernel repair: vertices it visits
-    uint32_t pad;
+    uint32_t fault;        // a barrier gave up: no field says anything about the graph
     unsigned long long sym;   // nonzero: some graph's first-sweep checksum was not 0
     unsigned long long live;  // first sweep's live entries
     unsigned long long swept[2];  // live entries and vertices visited by the sweeps so far
@@ -49,8 +49,8 @@ enum : uint32_t { SWEEP_ELSEWHERE = 0, SWEEP_GRID = 1, SWEEP_TAIL = 2 };
 struct GridBar {
     unsigned long long count;  // arrivals of this launch
     unsigned long long gen;    // serial sections of this launch that ended
-    uint32_t left;             // blocks that left
-    uint32_t failed;
+    uint32_t left;             // blocks that left; in the high half, those a barrier gave up on
+    uint32_t failed;           // a barrier of this launch gave up
 };
 
 // Per-sweep work state: warp items for rows longer than SWEEP_TINY, per-vertex
@@ -179,7 +179,8 @@ void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start
                          const cudaGraphConditionalHandle* cond);
 void launch_query(const uint16_t* snap, uint32_t n, const uint32_t* v, uint16_t* out, uint32_t k, cudaStream_t s);
 // First-fit coloring of list[0, m) in list order. `place`: n words, `rows`:
-// kColorWords words of scratch; `colored` receives how many had no color.
+// kColorWords words of scratch; `colored` receives how many had no color
+// (NONE32: a barrier gave up, the list is colored in part).
 constexpr uint32_t kColorWindow = 128;  // vertices gathered at once
 constexpr uint32_t kColorWords = kColorWindow * (64 + kColorWindow / 32);
 void launch_color_list(const Dev& g, const uint32_t* list, uint32_t m, uint32_t* place, uint32_t* rows, GridBar* bar,
