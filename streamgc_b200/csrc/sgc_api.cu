@@ -178,7 +178,7 @@ int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool tim
         launch_repair_begin(h->g, h->sb, mode, h->num_sms, h->stream);
         h->launches += (mode == SWEEP_INDEP && h->g.touched) ? 2 : 1;
     } else {
-        launch_repair_fused(h->g, h->sb, &in, h->num_sms, h->stream, nullptr);
+        launch_repair_fused(h->g, h->sb, &in, h->stream, nullptr);
         h->launches += 1;
         TRY(check_cuda("repair"));
         TRY(read_back());
@@ -198,7 +198,7 @@ int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool tim
         launch_repair_step(h->g, h->sb, h->num_sms, h->stream, nullptr);
         h->launches += 1 + (mode == SWEEP_INDEP ? 6 : 4) + 3;
         if (!timed) {
-            launch_repair_fused(h->g, h->sb, nullptr, h->num_sms, h->stream, nullptr);
+            launch_repair_fused(h->g, h->sb, nullptr, h->stream, nullptr);
             h->launches += 1;
         }
         TRY(read_back());
@@ -388,6 +388,7 @@ int sgci::create_internal(const StreamGCConfig* cfg, const sgc_options* opt_in, 
     std::vector<uint32_t> hdmap(n, EMPTY);
     std::vector<uint32_t> hw(n, 0);
     uint32_t num_hd = 0;
+    uint64_t sweep_items = 0;  // work items of a sweep over every row filled to capacity
     for (uint32_t x = 0; x < n; x++) {
         if (row_ptr[x + 1] < row_ptr[x]) return fail(SGC_EINVAL, "row_ptr not monotone at %u", x);
         const uint64_t cnt64 = row_ptr[x + 1] - row_ptr[x];
@@ -397,6 +398,7 @@ int sgci::create_internal(const StreamGCConfig* cfg, const sgc_options* opt_in, 
         const uint32_t cap = std::max<uint32_t>(cnt + extra, 8u);
         rp[x + 1] = rp[x] + cap;
         hw[x] = cnt;
+        if (cap > SWEEP_TINY) sweep_items += (cap + opt.repair_tile - 1) / opt.repair_tile;
         const uint32_t thr = (ex && ex->thr_word) ? ex->thr_word[x >> 5] : cfg->histogram_threshold;
         if (degree[x] > thr) hdmap[x] = num_hd++;
     }
@@ -565,6 +567,7 @@ int sgci::create_internal(const StreamGCConfig* cfg, const sgc_options* opt_in, 
     A(&sb.bar, 1, 0);
     sb.tile = opt.repair_tile;
     sb.G = G;
+    sb.blocks = repair_blocks(n, sweep_items, h->num_sms);
     if (g.exact) A(&g.touched, (n + 31) / 32 + 1, 0);
     else g.touched = nullptr;
     if (g.exact && G == 1) {  // incremental snapshots (a batched handle publishes per graph)

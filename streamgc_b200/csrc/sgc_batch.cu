@@ -133,7 +133,7 @@ void enqueue_head(sgc_batch* b, cudaStream_t s, const cudaGraphConditionalHandle
                    &h->ctl->drain_n);
     launch_drain(h->g, &h->ctl->drain_n, (b->flags & SGC_BATCH_STREAM_ORDER) != 0, &h->ctl->drain_failed, s);
     const RepairIn in{(uint32_t)SWEEP_INDEP, 64u, 0u};
-    launch_repair_fused(h->g, h->sb, &in, h->num_sms, s, cond);
+    launch_repair_fused(h->g, h->sb, &in, s, cond);
 }
 
 void enqueue_tail(sgc_batch* b, cudaStream_t s) {

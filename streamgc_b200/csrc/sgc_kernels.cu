@@ -24,6 +24,8 @@
 #include <cuda_runtime.h>
 #include <cuda/atomic>
 
+#include <algorithm>
+
 #include "sgc_kernels.cuh"
 
 namespace sgc {
@@ -82,10 +84,10 @@ __device__ __forceinline__ void list_bits(uint32_t w, uint32_t bits, uint32_t* l
 // a warp each; chunks meet at a block barrier. The time is one warp's chain of
 // dependent loads and instructions. One warp alone, its words in L2, took 4.1 us
 // per update (8,192 updates of an R-MAT graph of 16,384 vertices, 34 ms); with
-// the searches prepared and the words in L1 0.9 us. Reading ahead without
+// the searches prepared and the words in L1 0.85 us. Reading ahead without
 // handing over the slots gave 2.4 us: the search's instructions, not only its
 // loads, are on the chain.
-__global__ void __launch_bounds__(32 * kSeqWarps, 1) seq_apply_kernel(Dev g, const EdgeUpdate* __restrict__ ups,
+__global__ void __launch_bounds__(32 * kSeqWarps, 2) seq_apply_kernel(Dev g, const EdgeUpdate* __restrict__ ups,
                                                                    const uint32_t* __restrict__ segs,
                                                                    const uint32_t* dyn, uint32_t n) {
     __shared__ SeqShared sh;
@@ -121,11 +123,12 @@ __global__ void __launch_bounds__(32 * kSeqWarps, 1) seq_apply_kernel(Dev g, con
 void launch_det_apply(const Dev& g, const EdgeUpdate* ups, uint32_t n, cudaStream_t s) {
     if (n) seq_apply_kernel<<<1, 32 * kSeqWarps, 0, s>>>(g, ups, nullptr, nullptr, n);
 }
+// A block per segment, but not one on every SM (spare_sms): the kernel is as long
+// as its longest segments.
 void launch_seg_apply(const Dev& g, const EdgeUpdate* ups, const uint32_t* segs, const uint32_t* dyn, uint32_t max_segs,
                       int num_sms, cudaStream_t s) {
-    uint32_t blocks = max_segs;
-    if (blocks > (uint32_t)num_sms * 4) blocks = num_sms * 4;
-    seq_apply_kernel<<<blocks ? blocks : 1, 32 * kSeqWarps, 0, s>>>(g, ups, segs, dyn, 0);
+    const uint32_t blocks = std::min(std::max(max_segs, 1u), spare_sms(num_sms));
+    seq_apply_kernel<<<blocks, 32 * kSeqWarps, 0, s>>>(g, ups, segs, dyn, 0);
 }
 
 __device__ __forceinline__ unsigned long long edge_key(uint32_t u, uint32_t v) {
@@ -1513,18 +1516,30 @@ void launch_repair_begin(const Dev& g, const SweepBufs& b, SweepMode mode, int n
 // Most repairs are short: an epoch's worklist of some ten thousand vertices, two
 // to ten sweeps of a few microseconds of work each. As fourteen launches per
 // sweep, and a host or while-node round trip, a sweep took 55 us (epochs of 4,096
-// updates on a mesh of 24,001 vertices: 245 us, now 152). One cooperative launch
-// with a block per SM runs the same passes with a barrier across the grid (2 us)
-// between them and leaves out the passes that have nothing to do; a short
-// worklist is left to kTailBlocks blocks, whose barrier costs less.
-//   kTailList, kTailItems: what sixteen blocks finish in one or two rounds of
-// their warps. Sweeps of a power-law graph of 2 M vertices there: 40 us against
-// 49 on the whole grid.
-//   kFusedMax: the passes share one register budget (80: 24 warps per SM), so a
-// sweep over many vertices, where the item passes' 40 warps per SM pay and a
-// launch costs little, is left to the kernels above.
-constexpr uint32_t kFusedThreads = 768;
+// updates on a mesh of 24,001 vertices: 245 us, now 142). One cooperative launch
+// runs the same passes with a barrier across the grid (2 us) between them and
+// leaves out the passes that have nothing to do; a short worklist is left to
+// kTailBlocks blocks, whose barrier costs less.
+//   kTailList, kTailItems: what sixteen blocks finish in a few rounds of their
+// warps. Sweeps of a power-law graph of 2 M vertices there: 40 us against 49 on
+// the whole grid.
+//   kFusedMax: a sweep over many vertices, where the item passes' 40 warps per SM
+// pay and a launch costs little, is left to the kernels above.
+//   kFusedThreads: a cooperative launch starts only when all its blocks have room,
+// so a block takes no more than half of an SM's registers (384 threads of 80) and
+// two handles' repairs, or one and another handle's stream-order apply, run side
+// by side. With 768 threads a publish of 157 us waited up to 7.7 ms for such an
+// apply, and two loads of a Chung-Lu graph of 300,007 vertices at once took 6.3 ms
+// each, now 4.7. Alone, sweeps of that load pay 2 % for the halved blocks.
+constexpr uint32_t kFusedThreads = 384;
 
+// A thread per vertex and a warp per work item of the rows when full is as much as
+// a sweep can use; never a block on every SM (spare_sms), and a few at least.
+uint32_t repair_blocks(uint64_t vertices, uint64_t items, int num_sms) {
+    const uint64_t want = std::max<uint64_t>((vertices + kFusedThreads - 1) / kFusedThreads,
+                                             (items + kFusedThreads / 32 - 1) / (kFusedThreads / 32));
+    return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(want, kTailBlocks), spare_sms(num_sms));
+}
 
 // The first `nb` blocks of the grid meet. A thread's writes before the barrier
 // are seen after it by plain loads in all of them. Round by round the arrivals
@@ -1758,7 +1773,7 @@ void launch_color_list(const Dev& g, const uint32_t* list, uint32_t m, uint32_t*
     cudaMemsetAsync(place, 0, (size_t)g.n * 4, s);
     list_places_kernel<<<num_sms, 256, 0, s>>>(list, m, place);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(num_sms);
+    cfg.gridDim = dim3(std::min(kColorWindow, spare_sms(num_sms)));  // a block per vertex of a window
     cfg.blockDim = dim3(kColorThreads);
     cfg.stream = s;
     cudaLaunchAttribute attr;
@@ -1801,7 +1816,7 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
         const uint32_t next = counted ? *b.next_items : NONE32;
         uint32_t go = SWEEP_ELSEWHERE;
         if (rc.cont && lim <= most) {
-            if (sync.nb > kTailBlocks) go = lim <= kTailList && next <= kTailItems ? SWEEP_TAIL : SWEEP_GRID;
+            if (sync.nb == gridDim.x) go = gridDim.x > kTailBlocks && lim <= kTailList && next <= kTailItems ? SWEEP_TAIL : SWEEP_GRID;
             else if (lim <= 4 * kTailList && next <= 4 * kTailItems) go = SWEEP_TAIL;  // else another launch goes on
         }
         rc.go = go;
@@ -1893,7 +1908,7 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
         lim = rc.lim;
     }
 }
-__global__ void __launch_bounds__(kFusedThreads, 1) repair_fused_kernel(Dev g, SweepBufs b, int start, RepairIn in,
+__global__ void __launch_bounds__(kFusedThreads, 2) repair_fused_kernel(Dev g, SweepBufs b, int start, RepairIn in,
                                                                         uint32_t most,
                                                                         cudaGraphConditionalHandle cond,
                                                                         int has_cond) {
@@ -1909,10 +1924,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) repair_fused_kernel(Dev g, S
     if (has_cond) cudaGraphSetConditional(cond, rc.cont);
 }
 
-void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start, int num_sms, cudaStream_t s,
+void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start, cudaStream_t s,
                          const cudaGraphConditionalHandle* cond) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(num_sms);
+    cfg.gridDim = dim3(b.blocks);
     cfg.blockDim = dim3(kFusedThreads);
     cfg.stream = s;
     cudaLaunchAttribute attr;

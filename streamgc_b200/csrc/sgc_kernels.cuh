@@ -63,6 +63,7 @@ struct SweepBufs {
     uint32_t G;                  // graphs of the handle (entries of g.gctl)
     RepairCtl* rc;
     GridBar* bar;
+    uint32_t blocks;             // of the one-kernel repair (repair_blocks)
     unsigned long long* acc_bm;  // OR of neighbor colors 1..64, per vertex
     uint32_t* acc_fl;            // bit0: a same-colored neighbor has higher priority
     uint32_t* pend_v;            // Jacobi commit list
@@ -133,7 +134,7 @@ void launch_conc_apply(const Dev& g, const EdgeUpdate* ups, uint32_t n, const Ed
 void launch_conc_apply_dyn(const Dev& g, const EdgeUpdate* ups, const uint32_t* dyn, const EdgeOrder& eo,
                            int num_sms, int blocks_per_sm, cudaStream_t s);
 int conc_apply_occupancy();
-// One warp per segment [segs[k], segs[k+1]), k < dyn[2]: each segment in stream order.
+// One block per segment [segs[k], segs[k+1]), k < dyn[2]: each segment in stream order.
 void launch_seg_apply(const Dev& g, const EdgeUpdate* ups, const uint32_t* segs, const uint32_t* dyn, uint32_t max_segs,
                       int num_sms, cudaStream_t s);
 void launch_dirty_list(const Dev& g, uint32_t* list, uint32_t* count, cudaStream_t s);
@@ -175,7 +176,13 @@ void launch_repair_step(const Dev& g, const SweepBufs& b, int num_sms, cudaStrea
 // above to go on where the next one visits more. With `cond`, that graph
 // conditional receives b.rc->cont.
 constexpr uint32_t kFusedMax = 1u << 19;
-void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start, int num_sms, cudaStream_t s,
+uint32_t repair_blocks(uint64_t vertices, uint64_t items, int num_sms);
+// The most blocks of a kernel that may run for milliseconds: a few SMs stay free
+// for kernels of other handles whose blocks need more of an SM than it leaves (the
+// pass over hub rows after a batch: 1,024 threads of 48 registers). With a block on
+// all 148, epochs of a mesh beside a load's repair waited up to 2.5 ms for it.
+inline uint32_t spare_sms(int num_sms) { return num_sms > 32 ? num_sms - 4 : num_sms; }
+void launch_repair_fused(const Dev& g, const SweepBufs& b, const RepairIn* start, cudaStream_t s,
                          const cudaGraphConditionalHandle* cond);
 void launch_query(const uint16_t* snap, uint32_t n, const uint32_t* v, uint16_t* out, uint32_t k, cudaStream_t s);
 // First-fit coloring of list[0, m) in list order. `place`: n words, `rows`:

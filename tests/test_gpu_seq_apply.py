@@ -28,7 +28,7 @@ def hot_updates(n, count, seed, out_of_range):
 SHAPES = [(2, 1, 0, 64), (7, 3, 0, 2), (40, 20, 100, 8), (96, 70, 30, 64), (400, 300, 50, 64)]
 
 
-@pytest.mark.parametrize("count", [1, 14, 15, 16, 31, 4000])  # around the chunks of 15
+@pytest.mark.parametrize("count", [1, 8, 9, 10, 14, 15, 16, 19, 31, 4000])  # around the chunks of 9
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"n{s[0]}")
 def test_hot_rows_match_the_oracle(shape, count):
     n, degree, slack, thr = shape
