@@ -376,16 +376,21 @@ __global__ void row_total_kernel(Dev g, unsigned long long* total) {
 // Every slot's edge as a key (lower endpoint << bits | higher), bit 2 * bits set
 // where the slot holds none. A warp takes 32 rows and their room in `keys` with
 // one atomic (one per entry, on one word, took 1.0 ms for 8 M entries), then
-// writes row by row.
+// writes row by row, four entries per lane in flight. Its rows lie as far apart as
+// there are warps: where low ids are the hubs, 32 consecutive rows were 2.3 ms on
+// one warp (R-MAT, 262,144 vertices).
 __global__ void __launch_bounds__(256) validate_kernel(Dev g, unsigned long long* keys, uint32_t bits,
                                                        unsigned long long* words /* uncolored, max color, oor, -, -, cursor */) {
+    constexpr uint32_t K = 4;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5, lane = lane_id();
     uint32_t bare = 0, top = 0;
     unsigned long long oor = 0;
-    for (uint32_t x0 = 32 * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); x0 < g.n; x0 += 32 * warps) {
-        const uint32_t mine = x0 + lane < g.n ? row_len(g, x0 + lane) : 0u;
-        const uint32_t color = x0 + lane < g.n ? color_of(g.st[x0 + lane]) : 0u;
-        const unsigned long long start = x0 + lane < g.n ? g.rp[x0 + lane] : 0ull;
+    for (uint64_t x0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x0 < g.n; x0 += 32ull * warps) {
+        const uint64_t own = x0 + (uint64_t)lane * warps;
+        const bool in = own < g.n;
+        const uint32_t mine = in ? row_len(g, (uint32_t)own) : 0u;
+        const uint32_t color = in ? color_of(g.st[own]) : 0u;
+        const unsigned long long start = in ? g.rp[own] : 0ull;
         top = color > top ? color : top;
         unsigned long long upto = mine;
         for (int off = 1; off < 32; off <<= 1) {
@@ -395,22 +400,28 @@ __global__ void __launch_bounds__(256) validate_kernel(Dev g, unsigned long long
         unsigned long long base = 0;
         if (lane == 31 && upto) base = atomicAdd(words + 5, upto);
         base = __shfl_sync(FULL, base, 31);
-        for (uint32_t k = 0; k < 32 && x0 + k < g.n; k++) {
-            const uint32_t x = x0 + k, len = __shfl_sync(FULL, mine, k);
+        for (uint32_t k = 0; k < 32 && x0 + (uint64_t)k * warps < g.n; k++) {
+            const uint32_t x = (uint32_t)(x0 + (uint64_t)k * warps), len = __shfl_sync(FULL, mine, k);
             const unsigned long long s = __shfl_sync(FULL, start, k), out = base + __shfl_sync(FULL, upto, k) - len;
             bool any = false;
-            for (uint32_t j = lane; j < len; j += 32) {
-                const uint32_t y = g.col[s + j];
-                unsigned long long key = 1ull << (2 * bits);
-                if (y != INV && !(g.blen && (y & TOMB))) {  // not a free slot or deleted run entry
-                    if (y >= g.n) {
-                        oor++;
-                    } else {
-                        any = true;
-                        key = x < y ? ((unsigned long long)x << bits) | y : ((unsigned long long)y << bits) | x;
+            for (uint32_t j = lane; j < len; j += 32 * K) {
+                uint32_t y[K];
+#pragma unroll
+                for (uint32_t t = 0; t < K; t++) y[t] = j + 32 * t < len ? g.col[s + j + 32 * t] : INV;
+#pragma unroll
+                for (uint32_t t = 0; t < K; t++) {
+                    if (j + 32 * t >= len) break;
+                    unsigned long long key = 1ull << (2 * bits);
+                    if (y[t] != INV && !(g.blen && (y[t] & TOMB))) {  // not a free slot or deleted run entry
+                        if (y[t] >= g.n) {
+                            oor++;
+                        } else {
+                            any = true;
+                            key = x < y[t] ? ((unsigned long long)x << bits) | y[t] : ((unsigned long long)y[t] << bits) | x;
+                        }
                     }
+                    keys[out + j + 32 * t] = key;
                 }
-                keys[out + j] = key;
             }
             if (__any_sync(FULL, any) && lane == k && color == 0) bare++;
         }

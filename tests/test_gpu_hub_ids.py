@@ -51,3 +51,7 @@ def test_forced_compaction(graphs):
     near, apart = times(graphs, step)
     assert near < 2 * apart, (near, apart)
 
+
+def test_validator(graphs):
+    near, apart = times(graphs, lambda h, edges: h.validate)
+    assert near < 2 * apart, (near, apart)
