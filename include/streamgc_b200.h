@@ -47,8 +47,10 @@ typedef struct sgc_handle sgc_handle;
 /* On handles with SGC_OPT_PROFILE a repair runs each sweep's passes as kernels
  * of their own and times them, a host synchronization per sweep. With
  * SGC_OPT_EXACT_SELECT this flag keeps a publish after concurrent batches to the
- * one kernel that runs the whole loop otherwise, one host synchronization per
- * epoch: those sweeps are not timed (sgc_stats.sweep_ms stays 0). */
+ * one kernel that runs the whole loop otherwise: those sweeps are not timed
+ * (sgc_stats.sweep_ms stays 0). On every handle such a publish returns after its
+ * snapshot is written, with one host synchronization per epoch that covers both;
+ * without the flag the snapshot follows in stream order. */
 #define SGC_OPT_GRAPH_PUBLISH 4u
 /* With SGC_OPT_EXACT_SELECT, compaction also sorts every row of at most 1024
  * live entries into one base run, and compacts a row whose unsorted tail (the

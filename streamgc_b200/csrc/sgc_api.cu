@@ -121,10 +121,10 @@ int set_clean(sgc_handle* h, uint32_t v) {
     return SGC_OK;
 }
 
-// Writes the back half of the snapshot and makes it the front. With
-// incremental snapshots only the colors changed in the last two epochs are
-// copied (plus a full copy while snap_full says so).
-void publish_snapshot(sgc_handle* h) {
+// Writes the back half of the snapshot. With incremental snapshots only the
+// colors changed in the last two epochs are copied (plus a full copy while
+// snap_full says so).
+void write_snapshot(sgc_handle* h) {
     const int back = 1 - h->front;
     if (h->g.chg) {
         launch_snapshot_changes(h->g, h->chg_prev, h->snap[back], h->stream);
@@ -135,7 +135,12 @@ void publish_snapshot(sgc_handle* h) {
         h->launches += 1;
         if (h->snap_full > 0) h->snap_full--;
     }
-    h->front = back;
+}
+
+// Writes the back half and makes it the front.
+void publish_snapshot(sgc_handle* h) {
+    write_snapshot(h);
+    h->front = 1 - h->front;
 }
 
 // Tier-1 loop of run_conflict_repair (streamgc.cu:1317-1393) on compact rows,
@@ -152,7 +157,9 @@ void publish_snapshot(sgc_handle* h) {
 //   `timed`: each sweep's passes as kernels of their own with events between
 //   them (SGC_OPT_PROFILE); otherwise the loop runs in one cooperative kernel
 //   except for sweeps over many vertices.
-int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool timed) {
+//   `snapshot`: the back half is written behind that kernel, so that one wait
+//   covers both, and again where other sweeps or Tier-2 changed colors since.
+int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool timed, bool snapshot) {
     const bool indep = h->g.exact != 0;
     const SweepMode mode = indep ? SWEEP_INDEP : SWEEP_TIER1;
     const uint32_t every = h->opt.full_repair_every;
@@ -180,9 +187,11 @@ int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool tim
     } else {
         launch_repair_fused(h->g, h->sb, &in, h->stream, nullptr);
         h->launches += 1;
+        if (snapshot) write_snapshot(h);
         TRY(check_cuda("repair"));
         TRY(read_back());
     }
+    bool rewrite = snapshot && rc->cont;
     for (uint32_t sweeps = 0; timed || rc->cont; sweeps++) {
         if (sweeps > in.max_sweeps) return fail(SGC_EDEVICE, "repair loop ran past %u sweeps", in.max_sweeps);
         sgc_handle::SweepEvents se{};
@@ -206,6 +215,12 @@ int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool tim
     }
     TRY(check_cuda("repair"));
     TRY(finish_repair(h, rep));
+    rewrite |= snapshot && rep->tier2_ran;
+    if (rewrite) {
+        launch_snapshot(h->g, h->snap[1 - h->front], h->stream);
+        h->launches += 1;
+        TRY(sync(h));
+    }
     if (h->opt.flags & (SGC_OPT_PROFILE | SGC_OPT_GRAPH_PUBLISH)) h->sweep_bytes += 8ull * rc->swept[0] + 28ull * rc->swept[1];
     return SGC_OK;
 }
@@ -802,7 +817,7 @@ int sgc_repair(sgc_handle* h, sgc_repair_report* rep) {
     TRY(drain(h, h->last_mode == SGC_MODE_DETERMINISTIC, &h->ctl->drain_failed));
     // drain_and_compact's rebuild is subsumed: the first (full) sweep rebuilds every bitmap first.
     TRY(read_drain(h, &r, before));
-    TRY(repair_loop(h, &r, true, true));
+    TRY(repair_loop(h, &r, true, true, false));
     if (rep) *rep = r;
     return SGC_OK;
 }
@@ -810,13 +825,19 @@ int sgc_repair(sgc_handle* h, sgc_repair_report* rep) {
 int sgc_publish(sgc_handle* h, sgc_repair_report* rep) {
     if (!h) return fail(SGC_EINVAL, "null handle");
     CK(cudaSetDevice(h->device));
-    // SGC_OPT_GRAPH_PUBLISH: sweeps are not timed one by one
+    // SGC_OPT_GRAPH_PUBLISH: sweeps are not timed one by one, and the snapshot is
+    // written when the call returns
     const bool whole = (h->opt.flags & SGC_OPT_GRAPH_PUBLISH) && h->g.exact && h->last_mode == SGC_MODE_CONCURRENT;
     sgc_repair_report r{};
     TRY(compact_dirty(h, false));
     TRY(drain(h, h->last_mode == SGC_MODE_DETERMINISTIC, &h->ctl->drain_failed));
-    TRY(repair_loop(h, &r, false, !whole));
-    publish_snapshot(h);
+    const int e = repair_loop(h, &r, false, !whole, whole);
+    if (e != SGC_OK) {
+        if (whole) h->snap_full = 2;  // the change marks moved on with a half that is not published
+        return e;
+    }
+    if (whole) h->front = 1 - h->front;
+    else publish_snapshot(h);
     h->epochs++;
     if (rep) *rep = r;
     return check_cuda("publish");

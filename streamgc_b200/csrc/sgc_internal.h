@@ -149,7 +149,7 @@ int sync(sgc_handle* h);
 int compact_dirty(sgc_handle* h, bool force);
 int drain(sgc_handle* h, bool ordered, unsigned long long* failed_counter);
 int set_clean(sgc_handle* h, uint32_t v);
-int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool timed);
+int repair_loop(sgc_handle* h, sgc_repair_report* rep, bool force_full, bool timed, bool snapshot);
 int check_repair(const RepairCtl& rc);
 int finish_repair(sgc_handle* h, sgc_repair_report* rep);
 int apply_device(sgc_handle* h, const EdgeUpdate* src, uint32_t n, int mode);

@@ -36,7 +36,7 @@ static Rows ring(uint32_t n) {
     for (uint32_t v = 0; v < n; v++) adj[v] = {v ? v - 1 : n - 1, v + 1 < n ? v + 1 : 0};
     return Rows(adj);
 }
-static sgc_handle* make(const Rows& r) {
+static sgc_handle* make(const Rows& r, uint32_t flags = SGC_OPT_EXACT_SELECT) {
     StreamGCConfig cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.num_vertices = r.n;
@@ -45,7 +45,7 @@ static sgc_handle* make(const Rows& r) {
     cfg.histogram_threshold = 64;
     sgc_options o;
     sgc_default_options(&o);
-    o.flags = SGC_OPT_EXACT_SELECT;
+    o.flags = flags;
     sgc_handle* h = nullptr;
     CHECK(sgc_create_ex(&cfg, &o, r.ptr.data(), r.col.data(), r.deg.data(), &h) == SGC_OK);
     return h;
@@ -89,7 +89,32 @@ static void give_up() {
     CHECK(sgc_publish(h, &rep) == SGC_OK && rep.proper == 1 && rep.incremental == 0);
     sgc_destroy(h);
 
-    std::vector<uint32_t> ptr32(r.ptr.begin(), r.ptr.end());
+    // the publish that writes its snapshot before it waits: a half written behind a
+    // repair that gave up is not published, and both halves are whole afterwards
+    h = make(r, SGC_OPT_EXACT_SELECT | SGC_OPT_GRAPH_PUBLISH);
+    CHECK(sgc_publish(h, &rep) == SGC_OK);
+    for (uint32_t k = 0; k < 12; k++) {
+        std::vector<EdgeUpdate> ups(200);
+        for (uint32_t i = 0; i < ups.size(); i++) {
+            std::memset(&ups[i], 0, sizeof(EdgeUpdate));
+            ups[i].u = (k * 977 + i * 13) % r.n;
+            ups[i].v = (k * 389 + i * 29 + 7) % r.n;
+            ups[i].type = SGC_UPDATE_ADD;
+        }
+        CHECK(sgc_apply(h, ups.data(), (uint32_t)ups.size(), SGC_MODE_CONCURRENT) == SGC_OK);
+        CHECK(sgc_download(h, SGC_DL_SNAPSHOT, before.data(), 2ull * r.n) == SGC_OK);
+        if (k % 3 == 1) {
+            set_failed(h);
+            CHECK(sgc_publish(h, &rep) == SGC_EDEVICE);
+            CHECK(sgc_download(h, SGC_DL_SNAPSHOT, after.data(), 2ull * r.n) == SGC_OK && before == after);
+        } else {
+            CHECK(sgc_publish(h, &rep) == SGC_OK && rep.proper == 1);
+            CHECK(sgc_download(h, SGC_DL_COLORS, before.data(), 2ull * r.n) == SGC_OK);
+            CHECK(sgc_download(h, SGC_DL_SNAPSHOT, after.data(), 2ull * r.n) == SGC_OK && before == after);
+        }
+    }
+    sgc_destroy(h);
+
     for (uint32_t flags : {SGC_BATCH_CUDA_GRAPH, 0u}) {
         sgc_batch_graph gr[2];
         std::memset(gr, 0, sizeof(gr));

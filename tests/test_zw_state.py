@@ -117,9 +117,9 @@ def test_sorted_rows_keep_one_run():
 
 @pytest.mark.parametrize("name", ["delaunay2k", "rmat11"])
 def test_graph_publish_is_proper_and_keeps_invariants(name):
-    """The captured-graph publish (SGC_OPT_GRAPH_PUBLISH): every published
-    snapshot proper, the rows' invariants kept, the same counters advancing as
-    with the eager publish."""
+    """The publish that returns with its snapshot written (SGC_OPT_GRAPH_PUBLISH):
+    every published snapshot proper, the rows' invariants kept, the same counters
+    advancing as with the publish whose snapshot follows in stream order."""
     c = MG.build_case(name)
     g = S.Graph(c["rp"], c["col"], c["deg"])
     ups = np.concatenate([c["init"], c["bench"]])
@@ -138,6 +138,35 @@ def test_graph_publish_is_proper_and_keeps_invariants(name):
         assert v["violations"] == 0 and v["uncolored_with_edges"] == 0
         st = h.stats()
         assert st["epochs"] >= len(ups) // B and st["tier1_sweeps"] >= st["epochs"]
+
+
+def test_graph_publish_returns_with_its_snapshot():
+    """Nothing is left on the handle's stream when such a publish returns, with
+    sweeps left to other kernels (over 2^19 vertices) and without. On a handle
+    with SGC_OPT_PROFILE its sweeps are not timed, and it leaves what a publish
+    without the flag leaves."""
+    import torch
+    for n in (3000000, 70001):
+        v = np.arange(n)
+        e = np.concatenate([np.stack([v, (v + d) % n], 1) for d in (1, 2, 7)])
+        g = S.Graph.from_edges(n, e)
+        pick = e[:: max(1, n // 4000)]
+        ups = [S.updates_from(pick, np.full(len(pick), kind)) for kind in (1, 0)]
+        with S.StreamGC(g, exact_select=True, profile=True, graph_publish=True) as a, \
+                S.StreamGC(g, exact_select=True, profile=True) as b:
+            stream = torch.cuda.ExternalStream(a.cuda_stream())
+            for k in range(6):
+                for h in (a, b):
+                    h.apply(ups[k % 2], S.MODE_CONCURRENT)
+                a.synchronize()
+                timed = a.stats()["sweep_ms"]
+                assert a.publish()["proper"] == 1
+                assert stream.query()
+                assert b.publish()["proper"] == 1
+                assert a.stats()["sweep_ms"] == timed and b.stats()["sweep_ms"] > 0
+                assert np.array_equal(a.snapshot(), a.colors())
+                if k == 0:  # deletes only: no two updates race for a color
+                    assert np.array_equal(a.colors(), b.colors())
 
 
 def test_ingest_ring_matches_direct_applies():
