@@ -1037,8 +1037,10 @@ int sgc_color_core(sgc_handle* h, uint32_t min_degree, uint32_t* colored) {
     CK(cudaMemcpyAsync(deg.data(), h->g.deg, (size_t)h->n * 4, cudaMemcpyDeviceToHost, h->stream));
     TRY(sync(h));
     std::vector<uint32_t> list;
-    for (uint32_t x = 0; x < h->n; x++)
-        if (deg[x] >= min_degree && deg[x] > 0) list.push_back(x);
+    const uint32_t n = h->n, least = std::max(min_degree, 1u);
+    const uint32_t* dv = deg.data();
+    for (uint32_t x = 0; x < n; x++)
+        if (dv[x] >= least) list.push_back(x);
     std::sort(list.begin(), list.end(), [&](uint32_t a, uint32_t b) { return deg[a] != deg[b] ? deg[a] > deg[b] : a < b; });
     uint32_t done = 0;
     if (!list.empty()) {
@@ -1046,7 +1048,7 @@ int sgc_color_core(sgc_handle* h, uint32_t min_degree, uint32_t* colored) {
         CK(cudaMemcpyAsync(d, list.data(), list.size() * 4, cudaMemcpyHostToDevice, h->stream));
         launch_color_list(h->g, d, (uint32_t)list.size(), h->t2.rev_start, h->color_rows, h->sb.bar, h->t2.count,
                           h->num_sms, h->stream);
-        h->launches += 1;
+        h->launches += 2;
         CK(cudaMemcpyAsync(h->h_small, h->t2.count, 4, cudaMemcpyDeviceToHost, h->stream));
         for (uint32_t k = 0; k < std::max<uint32_t>(h->sb.G, 1u); k++)  // every graph's next repair is full
             CK(cudaMemsetAsync(&h->g.gctl[k].clean, 0, 4, h->stream));
