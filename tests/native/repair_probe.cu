@@ -1,5 +1,8 @@
 // Drives the library's internals where the public calls cannot reach a state:
 //   status   a control block that a repair gave up on, through finish_repair (no GPU)
+//   lists    repairs that start from a list of the test's own: only the winners of
+//            their conflicts, and a list that becomes short and grows again; as one
+//            kernel and as separate ones
 //   give_up  a barrier that gives up at once (its failure word is set before the
 //            call), through publish, core coloring and a batch's ticks
 // Exits 0 when everything was as it should be.
@@ -65,6 +68,95 @@ static void status() {
     rc.fault = 1;
     rep = {};
     CHECK(sgci::finish_repair(&h, &rep) == SGC_EDEVICE && rep.proper == 0);
+}
+
+// A repair under the independent-set rule of `states` from the worklist `list`,
+// as one kernel (as far as it goes) or pass by pass. Returns how often the one
+// kernel left a sweep to the others.
+static uint32_t repair_from(sgc_handle* h, const std::vector<uint32_t>& states, const std::vector<uint32_t>& list,
+                            bool fused, std::vector<uint32_t>& st, std::vector<uint64_t>& bm, sgc::RepairCtl& rc) {
+    CHECK(sgc_upload(h, SGC_DL_STATES, states.data(), 4ull * h->n) == SGC_OK);
+    rc = {};
+    rc.mode = sgc::SWEEP_INDEP;
+    rc.max_sweeps = 64;
+    rc.list = rc.it = rc.cont = 1;
+    const uint32_t count = (uint32_t)list.size();
+    CHECK(cudaMemcpy(h->sb.rc, &rc, sizeof(rc), cudaMemcpyHostToDevice) == cudaSuccess);
+    CHECK(cudaMemcpy(h->sb.wl, list.data(), 4ull * count, cudaMemcpyHostToDevice) == cudaSuccess);
+    CHECK(cudaMemcpy(h->sb.wl_count, &count, 4, cudaMemcpyHostToDevice) == cudaSuccess);
+    uint32_t left = 0;
+    for (uint32_t k = 0; k < 70; k++) {
+        if (fused) sgc::launch_repair_fused(h->g, h->sb, nullptr, h->stream, nullptr);
+        CHECK(cudaMemcpyAsync(&rc, h->sb.rc, sizeof(rc), cudaMemcpyDeviceToHost, h->stream) == cudaSuccess);
+        CHECK(cudaStreamSynchronize(h->stream) == cudaSuccess && !rc.fault);
+        if (!rc.cont) break;
+        left++;
+        sgc::launch_repair_sweep(h->g, h->sb, sgc::SWEEP_INDEP, h->num_sms, h->stream);
+        sgc::launch_repair_step(h->g, h->sb, h->num_sms, h->stream, nullptr);
+    }
+    CHECK(cudaGetLastError() == cudaSuccess && !rc.cont && rc.done);
+    st.resize(h->n);
+    bm.resize(h->n);
+    CHECK(sgc_download(h, SGC_DL_STATES, st.data(), 4ull * h->n) == SGC_OK);
+    CHECK(sgc_download(h, SGC_DL_BITMAPS, bm.data(), 8ull * h->n) == SGC_OK);
+    return left;
+}
+// Both ways from the same start; the result is proper and the same.
+static uint32_t both_ways(sgc_handle* h, const std::vector<uint32_t>& states, const std::vector<uint32_t>& list) {
+    std::vector<uint64_t> start(h->n), bm1, bm2;
+    std::vector<uint32_t> st1, st2;
+    sgc::RepairCtl rc1, rc2;
+    CHECK(sgc_download(h, SGC_DL_BITMAPS, start.data(), 8ull * h->n) == SGC_OK);
+    const uint32_t left = repair_from(h, states, list, true, st1, bm1, rc1);
+    sgc_validation v;
+    CHECK(sgc_validate(h, &v) == SGC_OK && v.violations == 0 && v.uncolored_with_edges == 0);
+    CHECK(sgc_upload(h, SGC_DL_BITMAPS, start.data(), 8ull * h->n) == SGC_OK);
+    repair_from(h, states, list, false, st2, bm2, rc2);
+    CHECK(st1 == st2 && bm1 == bm2 && rc1.it == rc2.it && rc1.need == rc2.need && rc1.next == rc2.next);
+    return left;
+}
+static void lists() {
+    sgc_repair_report rep{};
+    // The winner y of a conflict with its neighbor x is listed, x is not: the first
+    // sweep marks x and finds nobody who has to move.
+    for (uint32_t n : {50u, 60000u, 400003u}) {
+        const Rows r = ring(n);
+        sgc_handle* h = make(r);
+        CHECK(sgc_publish(h, &rep) == SGC_OK);
+        std::vector<uint32_t> good(n);
+        CHECK(sgc_download(h, SGC_DL_STATES, good.data(), 4ull * n) == SGC_OK);
+        for (uint32_t pairs : {1u, 4u, 700u, 5000u}) {
+            if (10 * pairs > n) continue;
+            std::vector<uint32_t> states = good, list;
+            const uint32_t apart = n / pairs;
+            for (uint32_t i = 0; i < pairs; i++) {
+                const uint32_t x = i * apart + 3, y = x + 1;  // the same degree: the higher id wins
+                states[x] = states[y];
+                list.push_back(y);
+            }
+            for (int k = 0; k < 20; k++) CHECK(both_ways(h, states, list) == 0);
+        }
+        sgc_destroy(h);
+    }
+    // 20 winners push 2,000 vertices (few enough for the first blocks: ids 8 apart,
+    // so that no word of marks counts as crowded), which push 12,000 (too many).
+    std::vector<std::vector<uint32_t>> adj(16000);
+    auto join = [&](uint32_t a, uint32_t b) {
+        adj[a].push_back(b);
+        adj[b].push_back(a);
+    };
+    auto other = [](uint32_t k) { return 8 * (k / 7) + 1 + k % 7; };  // the ids between
+    for (uint32_t l = 0; l < 2000; l++) {
+        join(other(l % 20), 8 * l);
+        for (uint32_t m = 0; m < 6; m++) join(8 * l, other(20 + 6 * l + m));
+    }
+    const Rows r(adj);
+    sgc_handle* h = make(r);
+    CHECK(sgc_publish(h, &rep) == SGC_OK);
+    std::vector<uint32_t> list;
+    for (uint32_t w = 0; w < 20; w++) list.push_back(other(w));
+    CHECK(both_ways(h, std::vector<uint32_t>(r.n, 1u | 1u << 16), list) == 1);
+    sgc_destroy(h);
 }
 
 static void give_up() {
@@ -146,6 +238,7 @@ static void give_up() {
 int main(int argc, char** argv) {
     const char* what = argc > 1 ? argv[1] : "";
     if (!std::strcmp(what, "status")) status();
+    else if (!std::strcmp(what, "lists")) lists();
     else if (!std::strcmp(what, "give_up")) give_up();
     else return 2;
     return 0;

@@ -39,3 +39,42 @@ def test_same_as_the_separate_kernels(n, exact):
             part = churn[k * 4096:(k + 1) * 4096]
             a.apply(part, S.MODE_DETERMINISTIC)
             b.apply(part, S.MODE_DETERMINISTIC)
+
+
+@pytest.mark.parametrize("exact", [True, False], ids=["exact", "reference"])
+@pytest.mark.parametrize("n", [33, 2049, 40000, 250007, (1 << 19) - 1, (1 << 19) + 1])
+def test_same_from_conflicting_colors(n, exact):
+    """Colors drawn at random: many conflicts, sweeps that recolor in every size
+    of list from all vertices down to a few."""
+    g = graph(n, n)
+    with S.StreamGC(g, exact_select=exact, profile=True) as a, S.StreamGC(g, exact_select=exact) as b:
+        for top in (2, 12, 200):
+            states = np.random.default_rng(top).integers(0, top + 1, n).astype(np.uint32)
+            for h in (a, b):
+                h.upload("states", states)
+            ra, rb = a.publish(), b.publish()
+            assert ra == rb and rb["proper"] == 1
+            for what in ("states", "bitmaps", "snapshot"):
+                assert np.array_equal(getattr(a, what)(), getattr(b, what)()), (top, what)
+            assert b.stats()["device_error"] == 0
+
+
+@pytest.mark.parametrize("cuda_graph", [True, False])
+def test_batch_of_more_vertices_than_one_kernel_sweeps(cuda_graph):
+    """The first tick's sweeps visit more than 2^19 vertices: the loop goes on in
+    the captured while-node (or from the host). Each graph's colors are those it
+    gets alone."""
+    graphs = [graph(n, n) for n in (250007, 300001, 40000)]
+    alone = []
+    for g in graphs:
+        with S.StreamGC(g, exact_select=True) as h:
+            assert h.publish()["proper"] == 1
+            alone.append(h.snapshot())
+    b = S.Batch(graphs, epoch_sizes=[1024] * 3, cuda_graph=cuda_graph)
+    try:
+        b.close_epochs()
+        assert b.tick()["proper"] == 1
+        for k, want in enumerate(alone):
+            assert np.array_equal(b.snapshot(k), want), k
+    finally:
+        b.close()

@@ -1,5 +1,6 @@
-"""What a repair reports when a barrier across the grid gives up. The failure
-word of the barrier is set before the call, so its waits end at once."""
+"""The one-kernel repair in states that the public calls do not reach: started
+from lists of the test's own, and with a barrier across the grid that gives up
+(its failure word is set before the call, so its waits end at once)."""
 import os
 import shutil
 import subprocess
@@ -34,3 +35,8 @@ def test_a_given_up_repair_is_an_error(probe):
 @pytest.mark.gpu
 def test_publish_core_coloring_and_ticks_report_it_and_recover(probe):
     probe("give_up")
+
+
+@pytest.mark.gpu
+def test_lists_of_winners_and_lists_that_grow_again(probe):
+    probe("lists")
