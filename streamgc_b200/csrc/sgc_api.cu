@@ -568,22 +568,22 @@ int sgci::create_internal(const StreamGCConfig* cfg, const sgc_options* opt_in, 
     A(&sb.fac_v, n);
     sb.fac_count = &h->ctl->fac_count;
     sb.live = &h->ctl->live;
-    A(&sb.wmark, (n + 31) / 32 + 1, 0);
+    A(&sb.wmark, (n + 31) / 32 + 3, 0);  // read and cleared sixteen bytes at a time, as rbits and touched
     A(&sb.wl, n);
     A(&sb.wl_count, 4, 0);
     sb.next_items = sb.wl_count + 1;
     sb.seed_count = sb.wl_count + 2;
     A(&sb.swept, 2, 0);
-    A(&sb.needf, n, 0);
+    A(&sb.needf, (size_t)n + 15, 0);  // cleared sixteen bytes at a time
     A(&sb.need_v, n);
     A(&sb.need_count, 4, 0);
-    A(&sb.rbits, (n + 31) / 32 + 1, 0);
+    A(&sb.rbits, (n + 31) / 32 + 3, 0);
     A(&sb.rc, 1, 0);
     A(&sb.bar, 1, 0);
     sb.tile = opt.repair_tile;
     sb.G = G;
     sb.blocks = repair_blocks(n, sweep_items, h->num_sms);
-    if (g.exact) A(&g.touched, (n + 31) / 32 + 1, 0);
+    if (g.exact) A(&g.touched, (n + 31) / 32 + 3, 0);
     else g.touched = nullptr;
     if (g.exact && G == 1) {  // incremental snapshots (a batched handle publishes per graph)
         A(&g.chg, (n + 31) / 32 + 1, 0);

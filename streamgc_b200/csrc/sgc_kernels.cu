@@ -61,6 +61,7 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t& total) 
 
 // One warp's words of a bitmask as list entries, appended at *count.
 __device__ __forceinline__ void list_bits(uint32_t w, uint32_t bits, uint32_t* list, uint32_t* count) {
+    if (!__any_sync(FULL, bits)) return;
     uint32_t total = 0;
     const uint32_t off = warp_excl_scan(__popc(bits), total);
     uint32_t base = 0;
@@ -1310,16 +1311,45 @@ __device__ __forceinline__ void mark_items(const Dev& g, const SweepBufs& b, uin
 
 __global__ void __launch_bounds__(256) mark_items_kernel(Dev g, SweepBufs b) { mark_items(g, b, gridDim.x); }
 
+// A pass over the `nw` words of a bitmask by the first `nb` blocks: f(w, bits), a
+// word per lane and warp-collective, with the words cleared. With many words per
+// thread they are read sixteen bytes per lane, and 128 that are all zero skipped
+// together: a mask of 65.6 M vertices has 2 M words, most of them zero, which were
+// thirty-seven rounds of 55,296 threads. (Epochs of 32,768 updates on a Chung-Lu
+// graph of that size: 474 us, 422 with these passes, sixteen-byte clearing and the
+// short sweeps left to the whole grid, kTailWords.)
+template <class F>
+__device__ __forceinline__ void take_words(uint32_t* words, uint32_t nw, uint32_t nb, F f) {
+    const uint32_t threads = nb * blockDim.x;
+    if (nw <= 4 * threads) {
+        for (uint32_t base = spread_warp(nb) * 32; base < nw; base += threads) {
+            const uint32_t w = base + lane_id();
+            uint32_t bits = 0;
+            if (w < nw) {
+                bits = words[w];
+                if (bits) words[w] = 0;
+            }
+            f(w, bits);
+        }
+        return;
+    }
+    for (uint32_t base = spread_warp(nb) * 128; base < nw; base += 4 * threads) {
+        const uint32_t w = base + 4 * lane_id();
+        uint4 q = make_uint4(0, 0, 0, 0);
+        if (w < nw) q = *reinterpret_cast<const uint4*>(words + w);  // there is room for the last three
+        if (!__any_sync(FULL, q.x | q.y | q.z | q.w)) continue;
+        if (q.x | q.y | q.z | q.w) *reinterpret_cast<uint4*>(words + w) = make_uint4(0, 0, 0, 0);
+        f(w, q.x);
+        f(w + 1, q.y);
+        f(w + 2, q.z);
+        f(w + 3, q.w);
+    }
+}
+
 // The next worklist: the marked vertices; clears the marks.
 __device__ __forceinline__ void collect_marks(const Dev& g, const SweepBufs& b, uint32_t nb) {
-    const uint32_t nw = (g.n + 31) / 32;
-    for (uint32_t base = spread_warp(nb) * 32; base < nw; base += nb * blockDim.x) {
-        const uint32_t w = base + lane_id();
-        uint32_t bits = 0;
-        if (w < nw) {
-            bits = b.wmark[w];
-            if (bits) b.wmark[w] = 0;
-        }
+    take_words(b.wmark, (g.n + 31) / 32, nb, [&](uint32_t w, uint32_t bits) {
+        if (!__any_sync(FULL, bits)) return;
         list_bits(w, bits, b.wl, b.wl_count);
         // the work items they will make (asked for only of a short list: many marks
         // in one word count as too many, and cost no walk over their rows)
@@ -1330,7 +1360,7 @@ __device__ __forceinline__ void collect_marks(const Dev& g, const SweepBufs& b, 
         }
         k = __reduce_add_sync(FULL, k);
         if (k && lane_id() == 0) atomicAdd(b.next_items, k);
-    }
+    });
 }
 // (and the recolored bits, which nothing reads any more)
 __global__ void collect_marks_kernel(Dev g, SweepBufs b) {
@@ -1418,6 +1448,10 @@ __global__ void repair_begin_kernel(Dev g, SweepBufs b) { repair_begin(g, b); }
 // marks; the list's length goes to *count. Thread per 32-vertex word.
 __device__ __forceinline__ void seed_worklist(const Dev& g, const SweepBufs& b, uint32_t nb, uint32_t* count) {
     const uint32_t nw = (g.n + 31) / 32;
+    if (!g.gidw && !g.gctl[0].full) {  // one graph, its touched vertices
+        take_words(g.touched, nw, nb, [&](uint32_t w, uint32_t bits) { list_bits(w, bits, b.wl, count); });
+        return;
+    }
     for (uint32_t base = spread_warp(nb) * 32; base < nw; base += nb * blockDim.x) {
         const uint32_t w = base + lane_id();
         uint32_t bits = 0;
@@ -1533,6 +1567,8 @@ void launch_repair_begin(const Dev& g, const SweepBufs& b, SweepMode mode, int n
 //   kTailList, kTailItems: what sixteen blocks finish in a few rounds of their
 // warps. Sweeps of a power-law graph of 2 M vertices there: 40 us against 49 on
 // the whole grid.
+//   kTailWords: the marks that sixteen blocks read in four rounds (3.1 M vertices).
+// They read all of them every sweep; for 65.6 M vertices that were eighty rounds.
 //   kFusedMax: a sweep over many vertices, where the item passes' 40 warps per SM
 // pay and a launch costs little, is left to the kernels above.
 //   kFusedThreads: a cooperative launch starts only when all its blocks have room,
@@ -1542,6 +1578,7 @@ void launch_repair_begin(const Dev& g, const SweepBufs& b, SweepMode mode, int n
 // apply, and two loads of a Chung-Lu graph of 300,007 vertices at once took 6.3 ms
 // each, now 4.7. Alone, sweeps of that load pay 2 % for the halved blocks.
 constexpr uint32_t kFusedThreads = 384;
+constexpr uint32_t kTailWords = 4 * 4 * kTailBlocks * kFusedThreads;
 
 // A thread per vertex and a warp per work item of the rows when full is as much as
 // a sweep can use; never a block on every SM (spare_sms), and a few at least.
@@ -1794,6 +1831,13 @@ void launch_color_list(const Dev& g, const uint32_t* list, uint32_t m, uint32_t*
     cudaLaunchKernelEx(&cfg, color_list_kernel, g, list, m, (const uint32_t*)place, rows, bar, colored);
 }
 
+// The first `threads` threads of the grid: words [0, nw) of an array on a 16-byte
+// boundary with room for three more become zero.
+__device__ __forceinline__ void zero_words(uint32_t* words, uint32_t nw, uint32_t tid, uint32_t threads) {
+    for (uint64_t i = 4ull * tid; i < nw; i += 4ull * threads)
+        *reinterpret_cast<uint4*>(words + i) = make_uint4(0, 0, 0, 0);
+}
+
 // False: a barrier gave up.
 __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, GridSync& sync, int start,
                                              const RepairIn& in, uint32_t most) {
@@ -1802,11 +1846,9 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
     const uint32_t nw = (g.n + 31) / 32;
     if (start) {  // no marks, no vertex conflicted
         const uint32_t threads = gridDim.x * blockDim.x;
-        for (uint32_t w = tid; w < nw; w += threads) {
-            b.wmark[w] = 0;
-            b.rbits[w] = 0;
-        }
-        for (uint32_t x = tid; x < g.n; x += threads) b.needf[x] = 0;
+        zero_words(b.wmark, nw, tid, threads);
+        zero_words(b.rbits, nw, tid, threads);
+        zero_words(reinterpret_cast<uint32_t*>(b.needf), (g.n + 3) / 4, tid, threads);
     }
     auto reset = [&] {
         if (threadIdx.x == 0) {
@@ -1826,7 +1868,8 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
         const uint32_t next = counted ? *b.next_items : NONE32;
         uint32_t go = SWEEP_ELSEWHERE;
         if (rc.cont && lim <= most) {
-            if (sync.nb == gridDim.x) go = gridDim.x > kTailBlocks && lim <= kTailList && next <= kTailItems ? SWEEP_TAIL : SWEEP_GRID;
+            const bool tail = gridDim.x > kTailBlocks && nw <= kTailWords && lim <= kTailList && next <= kTailItems;
+            if (sync.nb == gridDim.x) go = tail ? SWEEP_TAIL : SWEEP_GRID;
             else if (lim <= 4 * kTailList && next <= 4 * kTailItems) go = SWEEP_TAIL;  // else another launch goes on
         }
         rc.go = go;
@@ -1864,7 +1907,7 @@ __device__ __forceinline__ bool repair_fused(const Dev& g, const SweepBufs& b, G
     bool recolored = false;  // bits set in b.rbits
     for (;;) {
         if (recolored)
-            for (uint32_t w = tid; w < nw; w += sync.nb * blockDim.x) b.rbits[w] = 0;
+            zero_words(b.rbits, nw, tid, sync.nb * blockDim.x);
         if (go == SWEEP_ELSEWHERE) return true;
         const bool list = rc.list != 0;
         if (go == SWEEP_TAIL && sync.nb > kTailBlocks) {

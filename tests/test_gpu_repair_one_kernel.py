@@ -78,3 +78,26 @@ def test_batch_of_more_vertices_than_one_kernel_sweeps(cuda_graph):
             assert np.array_equal(b.snapshot(k), want), k
     finally:
         b.close()
+
+
+# the marks read sixteen bytes per lane by the first blocks (over 786,432 vertices)
+# and by the whole grid (over 7,077,888), the last size the first blocks take
+# (3,145,728) and the next
+@pytest.mark.parametrize("n", [786465, 3145728, 3145729, 7077921])
+def test_same_with_masks_of_many_words(n):
+    v = np.arange(n)
+    g = S.Graph.from_edges(n, np.concatenate([np.stack([v, (v + d) % n], 1) for d in (1, 5)]))
+    with S.StreamGC(g, exact_select=True, profile=True, full_repair_every=0) as a, \
+            S.StreamGC(g, exact_select=True, full_repair_every=0) as b:
+        states = np.random.default_rng(n).integers(0, 4, n).astype(np.uint32)
+        for h in (a, b):
+            h.upload("states", states)
+        churn = g.churn_stream(3 * 3000, 50, 3)
+        last = S.updates_from(np.array([[n - 2, n - 1], [n - 1, 0]]), np.ones(2))  # the last word too
+        for k in range(4):
+            ra, rb = a.publish(), b.publish()
+            assert ra == rb and rb["incremental"] == (k > 0)
+            for what in ("states", "bitmaps", "snapshot"):
+                assert np.array_equal(getattr(a, what)(), getattr(b, what)()), (k, what)
+            for h in (a, b):
+                h.apply(np.concatenate([churn[k * 3000:(k + 1) * 3000], last]), S.MODE_DETERMINISTIC)
