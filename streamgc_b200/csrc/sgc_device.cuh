@@ -968,10 +968,11 @@ __device__ __forceinline__ void warp_apply(const Dev& g, uint32_t u, uint32_t v,
 // A row edited after it was searched is settled again from the slots edited
 // since (seq_settle), which the applying warp logs.
 
-// One warp applies, nine prepare: at 96 registers a block leaves half of its SM's
-// registers to other work (a one-kernel repair's block of another handle; with
-// sixteen warps that repair waited for the whole batch). 8,192 updates of an R-MAT
-// graph of 16,384 vertices: 6.9 ms, with sixteen warps 7.7, and 8.5 at 64 registers.
+// One warp applies, nine prepare: at 96 registers a block takes less than half of
+// its SM's registers and leaves room for other work (a one-kernel repair's block of
+// another handle; with sixteen warps that repair waited for the whole batch). 8,192
+// updates of an R-MAT graph of 16,384 vertices: 6.9 ms, with sixteen warps 7.7 (8.5
+// at 64 registers), with ten at 84 registers 7.4.
 constexpr uint32_t kSeqWarps = 10;
 constexpr uint32_t kSeqChunk = kSeqWarps - 1;  // updates between two block barriers: one per preparing warp
 constexpr uint32_t kSeqMarks = 2048;

@@ -85,10 +85,10 @@ __device__ __forceinline__ void list_bits(uint32_t w, uint32_t bits, uint32_t* l
 // a warp each; chunks meet at a block barrier. The time is one warp's chain of
 // dependent loads and instructions. One warp alone, its words in L2, took 4.1 us
 // per update (8,192 updates of an R-MAT graph of 16,384 vertices, 34 ms); with
-// the searches prepared and the words in L1 0.85 us. Reading ahead without
+// the searches prepared and the words in L1 0.84 us. Reading ahead without
 // handing over the slots gave 2.4 us: the search's instructions, not only its
 // loads, are on the chain.
-__global__ void __launch_bounds__(32 * kSeqWarps, 2) seq_apply_kernel(Dev g, const EdgeUpdate* __restrict__ ups,
+__global__ void __launch_bounds__(32 * kSeqWarps, 1) seq_apply_kernel(Dev g, const EdgeUpdate* __restrict__ ups,
                                                                    const uint32_t* __restrict__ segs,
                                                                    const uint32_t* dyn, uint32_t n) {
     __shared__ SeqShared sh;
