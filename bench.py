@@ -1039,8 +1039,8 @@ def main():
                     help="plain path, e2e: batches staged through the two ingest slots (copy of the next "
                          "batch overlapping this epoch's publish)")
     ap.add_argument("--eager-publish", dest="graph_publish", action="store_false",
-                    help="plain path: publish with one host round trip per repair sweep instead of replaying "
-                         "the one kernel of the whole loop (SGC_OPT_GRAPH_PUBLISH, the default)")
+                    help="plain path: publish with one host round trip per repair sweep instead of one per "
+                         "epoch, the whole loop in one kernel (SGC_OPT_GRAPH_PUBLISH, the default)")
     ap.add_argument("--graph-publish", dest="graph_publish", action="store_true", help=argparse.SUPPRESS)
     ap.add_argument("--epoch-size", type=int, default=32768,
                     help="plain path: updates per epoch (the large workload's sweep uses 4096, 32768, 262144)")

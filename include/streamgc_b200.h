@@ -230,15 +230,16 @@ int sgc_publish(sgc_handle* h, sgc_repair_report* rep);
  * *epochs (may be NULL). */
 int sgc_process_stream(sgc_handle* h, const EdgeUpdate* updates, uint64_t n, int mode, uint32_t* epochs);
 
-/* Point queries against the last published snapshot (host arrays). */
+/* Point queries against the last published snapshot (host arrays): one launch
+ * and one wait per 65,536 vertices, through pinned, device-mapped buffers that
+ * the handle keeps (384 KiB of host memory, no device memory). The first query
+ * on a handle allocates them; make it before any CUDA stream capture. */
 int sgc_query(sgc_handle* h, const uint32_t* vertices, uint16_t* colors, uint32_t n);
 
 /* Point queries exactly like sgc_query, for callers that must not allocate
- * device memory: sgc_query takes scratch from the CUDA allocator on each call,
- * which a serving thread whose tenants already fill their HBM budget, or a
- * latency-bound path that must not enter the allocator, cannot afford. This
- * variant calls no cudaMalloc, cudaFree or allocating routine; it stages the
- * vertex ids and colors in a fixed scratch array compiled into the library
+ * memory even once: sgc_query makes pinned buffers at a handle's first query.
+ * This variant calls no allocating routine and needs no buffers per handle; it
+ * stages the vertex ids and colors in a fixed scratch array compiled into the library
  * (384 KiB, held by every GPU that loads the library until the process exits).
  * At most SGC_QUERY_NOALLOC_MAX vertices per call; larger n is rejected with
  * SGC_EINVAL. The first call on a device looks up the scratch's device address
@@ -263,9 +264,10 @@ int sgc_color_core(sgc_handle* h, uint32_t min_degree, uint32_t* colored);
 /* FindAvailableColor(x) (color_select.cuh:93-115) on the current device state. */
 int sgc_find_color(sgc_handle* h, uint32_t x, uint16_t* color);
 
-/* check_coloring_valid, streamgc.cu:448-556. Slabs beyond 2^32 slots are
- * counted without the distinct-edge sort: each edge at its lower endpoint's
- * entry (the same counts when every entry has its mirror). */
+/* check_coloring_valid, streamgc.cu:448-556. Slabs beyond 2^32 - 2^28 slots, and
+ * rows of 2^31 entries or more together, are counted without the distinct-edge
+ * sort: each edge at its lower endpoint's entry (the same counts when every entry
+ * has its mirror). Allocates 16 bytes per row entry for the call otherwise. */
 int sgc_validate(sgc_handle* h, sgc_validation* out);
 /* Checks every row's layout invariants on the device (a debugging aid with no
  * reference counterpart); call between batches. */

@@ -900,12 +900,10 @@ int sgc_query(sgc_handle* h, const uint32_t* v, uint16_t* out, uint32_t k) {
 }  // extern "C"
 
 // ---- point queries that allocate nothing ----
-// sgc_query takes its device scratch from the stream-ordered allocator on every
-// call. A serving thread that answers queries while its tenants already fill
-// their HBM budget, or one that must not enter the allocator on a latency-bound
-// path, cannot do that; it queries through this fixed scratch compiled into the
-// library instead: one static array per GPU that loads the library, held until
-// the process exits. Vertex ids occupy words [0, MAX); the uint16 colors are
+// sgc_query makes pinned buffers at a handle's first query. A thread that must
+// not enter an allocator even then queries through this fixed scratch compiled
+// into the library instead: one static array per GPU that loads the library, held
+// until the process exits. Vertex ids occupy words [0, MAX); the uint16 colors are
 // packed after them.
 namespace {
 constexpr uint32_t QUERY_NOALLOC_MAX = SGC_QUERY_NOALLOC_MAX;
